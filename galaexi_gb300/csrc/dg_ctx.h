@@ -120,6 +120,10 @@ struct dg_ctx {
   long long launches = 0;
   int lines_grid = 0;      // blocks of the persistent line volume kernel (SMs x resident blocks), on first use
   int prolong_grid = 0;    // blocks of the persistent prolongation kernel of the mixed form, on first use
+  // FP64 form, block fixed-point kernels: log2 of the largest |M_d| of each element and direction
+  // (kFxNoScale: outside the range of the scales), and the basis as limbs (VolFxBasis)
+  gxc::DBuf<float> MetL;
+  gxc::DBuf<int> fxb;
   gxc::DBuf<int> S2E;      // [side][5]: master elem, master local side, slave elem, slave local side, flip (0-based)
   gxc::DBuf<double> wq;    // 1D quadrature weights (n)
   // tangent-linear operator (R = S = Dual<1>), set up on first use
@@ -180,9 +184,18 @@ struct NPTable {
   int (*relift)(dg_ctx*, cudaStream_t st);
 };
 
+// the fixed-point kernels of the FP64 form, in translation units of their own (dg_fx<NP>.cu)
+struct FxTable {
+  int (*configure)(const dg_ctx*);
+  // volume kernel of the split forms PI and KG (Gauss-Lobatto nodes)
+  int (*volume)(dg_ctx*, const double* U, const gx::Gas<double>& gas, gx::RKArgs rk, int rkmode, cudaStream_t st);
+};
+
 }  // namespace gxc
 
-#define GX_DECLARE_NP(NPV) extern const gxc::NPTable gx_np_table_##NPV;
+#define GX_DECLARE_NP(NPV)                   \
+  extern const gxc::NPTable gx_np_table_##NPV; \
+  extern const gxc::FxTable gx_fx_table_##NPV;
 GX_DECLARE_NP(2)
 GX_DECLARE_NP(3)
 GX_DECLARE_NP(4)

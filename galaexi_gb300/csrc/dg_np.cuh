@@ -9,6 +9,8 @@
 #ifndef GX_NP
 #error "define GX_NP before including dg_np.cuh"
 #endif
+#define GX_CAT2(a, b) a##b
+#define GX_CAT(a, b) GX_CAT2(a, b)
 
 namespace {
 
@@ -98,7 +100,9 @@ int configure() {
   int rc = cfg_vol<R, -1, 0>() | cfg_vol<R, -1, 1>() | cfg_lift_lines<R>();
   if constexpr (NP >= 3) {
     rc |= cfg_vol<R, 0, 0>() | cfg_vol<R, 0, 1>() | cfg_vol<R, 1, 0>() | cfg_vol<R, 1, 1>() | cfg_vol<R, 2, 0>() |
-          cfg_vol<R, 2, 1>() | cfg_vol<R, 3, 0>() | cfg_vol<R, 3, 1>() | cfg_vol<R, 4, 0>() | cfg_vol<R, 4, 1>();
+          cfg_vol<R, 2, 1>();
+    if constexpr (!std::is_same<R, double>::value)
+      rc |= cfg_vol<R, 3, 0>() | cfg_vol<R, 3, 1>() | cfg_vol<R, 4, 0>() | cfg_vol<R, 4, 1>();
     rc |= cfg_lines<R, 0>() | cfg_lines<R, 3>() | cfg_lines<R, 4>();
   }
   return rc ? DG_ERR_CUDA : DG_OK;
@@ -257,8 +261,11 @@ int rhs(dg_ctx* ctx, PrecData<R>& P, const double* U, gx::RKArgs rk, int rkmode,
           case DG_SPLIT_SD: vrc = vol<R, 0>(ctx, P, U, rk, rkmode, gas, st); break;
           case DG_SPLIT_MO: vrc = vol<R, 1>(ctx, P, U, rk, rkmode, gas, st); break;
           case DG_SPLIT_DU: vrc = vol<R, 2>(ctx, P, U, rk, rkmode, gas, st); break;
-          case DG_SPLIT_KG: vrc = vol<R, 3>(ctx, P, U, rk, rkmode, gas, st); break;
-          default: vrc = vol<R, 4>(ctx, P, U, rk, rkmode, gas, st); break;
+          default:
+            // KG and PI: the FP64 form in fixed point, the mixed form line by line
+            if constexpr (std::is_same<R, double>::value) vrc = GX_CAT(gx_fx_table_, GX_NP).volume(ctx, U, gas, rk, rkmode, st);
+            else vrc = ctx->cfg.split_dg == DG_SPLIT_KG ? vol<R, 3>(ctx, P, U, rk, rkmode, gas, st)
+                                                        : vol<R, 4>(ctx, P, U, rk, rkmode, gas, st);
         }
       } else {
         gxh::set_error("split form needs N >= 2");
@@ -447,7 +454,5 @@ int cfl(dg_ctx* ctx, const double* U, double cflS, double dflS, double kpr, cuda
 
 }  // namespace
 
-#define GX_CAT2(a, b) a##b
-#define GX_CAT(a, b) GX_CAT2(a, b)
 extern const gxc::NPTable GX_CAT(gx_np_table_, GX_NP) = {configure<double>, configure<float>, rhs_d, rhs_f, cfl,
                                                          stage_events, configure_t, rhs_t, configure_a, adj, relift};

@@ -1,0 +1,596 @@
+// k_volume_fx: the volume kernel of the FP64 form on Gauss-Lobatto nodes for the split forms PI and KG,
+// in block fixed-point arithmetic on the integer pipes (dg_fx.cuh).
+//
+// VolInt_splitForm (src/dg/volint.f90:211-353), the viscous volume integral (EvalTransformedDiffFlux3D,
+// flux.f90:619-697, with D_hat^T), SurfIntCons (surfint.t90:352-586), -1, the Jacobian and the LSERK-W2
+// stage (vector.f90:163-183).  What k_volume computes with 518 FP64 instructions per node (N=7) takes 47
+// here (viscous stresses, the Jacobian, the stage update); the rest runs on the integer pipes.
+//
+// Summation by parts on Gauss-Lobatto nodes brings every term of a line to one antisymmetric form.  With
+// Q(i,l) = w_i DVolSurf(l,i) (i != l), Q(i,l) = -Q(l,i):
+//   split form    w_i sum_l DVolSurf(l,i) F#(i,l)   = sum_l Q(i,l) F#(i,l)
+//   viscous part  w_i sum_l D_hat^T(l,i) f(l)       = sum_l Q(i,l) (f(i) + f(l))
+//   surface       w_i L_hat(i) F                    = F on the line's end nodes
+// so a pair's flux is formed once, G = Q(a,b) (F#(a,b) + f(a) + f(b)), added to node a and subtracted
+// from node b, and the face fluxes are added to the end nodes as they are; 1/w_i is applied at the end.
+//
+// Mapping: one element per block.  A warp holds whole lines of one direction.  For even n a thread owns the
+// nodes k and k + n/2 of its line (k < n/2): their own pair first, then the pairs with the thread s places
+// on, s = 1 .. (n/2-1)/2 (four pairs from two partner nodes), and for even n/2 two of the four pairs with the
+// thread n/4 places on, whose thread evaluates the other two: n-1 pairs per thread, each of the line's
+// n(n-1)/2 pairs once.  For odd n a thread owns one node and evaluates the pairs (i, i+d mod n),
+// d = 1 .. (n-1)/2.  A pair's G stays with its thread for the own node and reaches the partner's thread by
+// warp shuffles.  Against one thread per line this needs the accumulators of two nodes instead of n, and
+// against one node per thread half of the shared-memory reads.
+#pragma once
+#include "dg_fx.cuh"
+#include "dg_kernels.cuh"
+
+namespace gx {
+
+template <int NP> struct VolFx {
+  static constexpr int OWN = NP % 2 ? 1 : 2;                      // nodes of a line per thread
+  static constexpr int TPL = NP / OWN;                            // threads per line
+  static constexpr int LPW = 32 / TPL;                            // lines per warp
+  static constexpr int TPD = (NP * NP + LPW - 1) / LPW;           // warp tasks per direction
+  static constexpr int TPW = OWN == 1 && TPD > 1 ? 2 : 1;         // tasks of one warp per direction
+  static constexpr int NW = (TPD + TPW - 1) / TPW, NT = 32 * NW;  // warps and threads of a block
+  static constexpr int NPT = (NP * NP * NP + NT - 1) / NT;        // nodes per thread
+  // blocks per SM for 128 registers per thread (512 threads), where shared memory holds them
+  static constexpr int MINB = NP >= 9 ? 1 : (512 / NT < 16 ? 512 / NT : 16);
+  // shared-memory slots of n^3 words: rho, aux, u, v, w, p, then per direction the metric terms (3) and
+  // the viscous fluxes (4), overwritten by the direction's five sums
+  __host__ __device__ static constexpr int dslots(int parab) { return parab ? 7 : 5; }
+  __host__ __device__ static constexpr size_t smem(int parab) {
+    return sizeof(fx64) * (size_t)(6 + 3 * dslots(parab)) * NP * NP * NP;
+  }
+};
+template <int NP, typename R, int SPLIT, typename S> struct UseVolFx {
+  static constexpr bool v = std::is_same<R, double>::value && std::is_same<S, double>::value && NP >= 3 &&
+                            (SPLIT == DG_SPLIT_PI || SPLIT == DG_SPLIT_KG);
+};
+// what the kernel needs of the basis: limbs of Q(i,l) 2^62 at [l + n i] and of w_0/w_i 2^60
+template <int NP> struct VolFxBasis {
+  FxLimb Q[NP * NP], iw[NP];
+};
+// MetL[e][3]: log2 of the largest |M_d| (2-norm) of the element, or kFxNoScale where its geometry is outside
+// the range the scales are made for (2^-150 .. 2^150); such elements take the FP64 path
+constexpr float kFxNoScale = 1e9f;
+
+// shifts of one direction (see vol_fx_scales) and the scales of its three kinds of rows: mass, momentum, energy
+struct VolFxShift {
+  int hV, hq, hg, hp, hG, hE;  // left shifts of the products
+  int k0, km, kv;              // right shifts: g for the mass row, g for the momentum rows, V for KG's energy row
+  int St, kt, Sq, kq;          // viscous fluxes: shift of the product, then right shift (momentum, energy rows)
+  int sM, t[3];                // metric terms * 2^sM; sums * 2^t
+};
+struct VolFxScale {
+  VolFxShift d[3];
+  int s_rho, s_aux, s_p, s_vel, s_tau, s_tq, t[3], ok;
+};
+// largest magnitudes of the element: fx_mag words; X_U2: float bits of |u|^2
+enum { X_RHO, X_AUX, X_U2, X_P, X_TAU, X_TQ, X_F0, X_FM = X_F0 + 3, X_FE = X_FM + 3, X_NMAX = X_FE + 3,
+       X_RHOMIN = X_NMAX, X_PMIN, X_N };
+
+__device__ __forceinline__ float fx_lse(float a, float b) {
+  const float m = fmaxf(a, b);
+  return m + __log2f(exp2f(a - m) + exp2f(b - m));
+}
+// The scales of one element, by the first warp (lanes 0-2: one direction each).  L.. are log2 of bounds.
+// A pair's terms, in units of 8 Q F# (density row: 4 Q F#):  V = Ms.us, q = rho_s V, g = Q q;
+//   mass g;  momentum g us + 4 Q ps Ms + 8 Q fs;  energy g aux_s (+ 2 Q ps V for KG) + 8 Q fs.
+// Products are shifted to use the range up: V, q < 2^61.4, g and the rows' sums of terms < 2^60.4, so that a
+// node's sum over its partners (sum |Q| <= 3.92 for N <= 9, |Q| < 1) and its face flux (< 2^61) stay below
+// 2^63.  Smaller contributions are shifted right to the scale that the largest allows.
+template <int SPLIT, int PARAB>
+__device__ __forceinline__ void vol_fx_scales(const unsigned* mag, const float* MetL, VolFxScale& S, int lane) {
+  const int d = min(lane, 2);
+  bool ok = MetL[d] < 200.f;
+  for (int c = 0; c < X_NMAX; ++c) ok = ok && (c == X_U2 || mag[c] < ((c < X_TAU ? 1022u + 150u : 1022u + 600u) << 20));
+  const unsigned lowest = (1022u - 150u) << 20;
+  ok = ok && mag[X_RHOMIN] > lowest && mag[X_PMIN] > lowest && mag[X_AUX] > lowest && mag[X_U2] < 0x7b000000u;
+  ok = ok && (mag[X_RHO] >> 20) - (mag[X_RHOMIN] >> 20) <= 8 && (mag[X_P] >> 20) - (mag[X_PMIN] >> 20) <= 8;
+  const float Lr = fx_log2(mag[X_RHO]), La = fx_log2(mag[X_AUX]), Lp = fx_log2(mag[X_P]);
+  const float Lu = 0.5f * __log2f(__uint_as_float(mag[X_U2])) + 1e-4f, LM = ok ? MetL[d] : 0.f;
+  const float Lt = fx_log2(mag[X_TAU]) + 0.8f, Lq = fx_log2(mag[X_TQ]) + 0.8f;
+  const int ev = (int)floorf(Lu) + 1, eM = (int)floorf(LM) + 1;
+  const int s_rho = 61 - fx_exp(mag[X_RHO]), s_vel = 59 - ev, sM = 59 - eM;
+  const int s_tau = 59 - fx_exp(mag[X_TAU]), s_tq = 59 - fx_exp(mag[X_TQ]);
+  VolFxShift o;
+  o.sM = sM;
+  const float LV = 2.f + LM + Lu, Lqq = 1.f + Lr + LV;
+  o.hV = (int)floorf(61.4f - LV) - (sM + s_vel - 64);
+  const int sV = sM + s_vel - 64 + o.hV;
+  o.hq = (int)floorf(61.4f - Lqq) - (s_rho + sV - 64);
+  const int sq = s_rho + sV - 64 + o.hq;
+  const int sg = (int)floorf(60.4f - Lqq);
+  o.hg = sg - (sq - 2);
+  // momentum rows
+  float Lm = fx_lse(Lqq + 1.f + Lu, 4.f + Lp + LM);
+  if (PARAB) Lm = fx_lse(Lm, 4.f + LM + Lt);
+  const int tm = (int)floorf(fminf(60.4f - Lm, 58.f - fx_log2(mag[X_FM + d])));
+  const int spx = (int)floorf(59.9f - Lp);
+  o.hG = max(2, max(tm - (sg + s_vel - 64), tm + 2 - (spx + sM - 64)));
+  o.km = min(sg + s_vel - 64 + o.hG - tm, 63);
+  const int sp = tm + 2 - (sM - 64) - o.hG;
+  // energy row
+  float Le = Lqq + 1.f + La;
+  if (SPLIT == DG_SPLIT_KG) Le = fx_lse(Le, 2.f + Lp + LV);
+  if (PARAB) Le = fx_lse(Le, 4.f + LM + Lq);
+  const int t4 = (int)floorf(fminf(60.4f - Le, 58.f - fx_log2(mag[X_FE + d])));
+  const int he = SPLIT == DG_SPLIT_KG ? max(2, t4 + 65 - sp - sV) : 2;
+  // p and aux have one scale for the three directions
+  int s_p = min(61 - fx_exp(mag[X_P]), sp + 1), s_aux = min(61 - fx_exp(mag[X_AUX]), t4 - sg + 64 - he);
+#pragma unroll
+  for (int x = 1; x < 4; x <<= 1) {
+    s_p = min(s_p, __shfl_xor_sync(0xffffffffu, s_p, x));
+    s_aux = min(s_aux, __shfl_xor_sync(0xffffffffu, s_aux, x));
+  }
+  o.hp = sp + 2 - s_p;
+  o.hE = t4 - sg - s_aux + 64;
+  o.kv = SPLIT == DG_SPLIT_KG ? min(sp + sV - 64 + o.hE - t4 - 1, 63) : 0;
+  // viscous fluxes: 8 Q f at the rows' scales, from M tau / 2^64 and M tq / 2^64
+  const int ft = tm + 5 - o.hG - (sM + s_tau - 64), fq = t4 + 5 - o.hE - (sM + s_tq - 64);
+  o.St = max(1, ft); o.kt = min(o.St - ft, 63);
+  o.Sq = max(1, fq); o.kq = min(o.Sq - fq, 63);
+  // mass row
+  const int t0 = (int)floorf(fminf((float)sg, 59.f - fx_log2(mag[X_F0 + d])));
+  o.k0 = min(sg - t0, 63);
+  o.t[0] = t0; o.t[1] = tm; o.t[2] = t4;
+  auto in = [](int h) { return h >= 1 && h <= 31; };
+  ok = ok && in(o.hV) && in(o.hq) && in(o.hg) && in(o.hp) && in(o.hG) && in(o.hE) && o.km >= 0 && o.k0 >= 0 && o.kv >= 0;
+  if (PARAB) ok = ok && in(o.St) && in(o.Sq);
+  ok = __all_sync(0xffffffffu, ok);
+  int tr[3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    tr[r] = o.t[r];
+#pragma unroll
+    for (int x = 1; x < 4; x <<= 1) tr[r] = min(tr[r], __shfl_xor_sync(0xffffffffu, tr[r], x));
+  }
+  if (lane < 3) S.d[d] = o;
+  if (lane == 0) {
+    S.s_rho = s_rho; S.s_aux = s_aux; S.s_p = s_p; S.s_vel = s_vel; S.s_tau = s_tau; S.s_tq = s_tq;
+    S.t[0] = tr[0]; S.t[1] = tr[1]; S.t[2] = tr[2];
+    S.ok = ok;
+  }
+}
+
+// The same sums in FP64 for one node, from global memory: for elements whose values do not fit one scale
+// per quantity (infinities and NaN, magnitudes outside 2^+-150, densities or pressures that differ by more
+// than 2^8 within the element, which one scale would hold less exactly than FP64).
+template <int NP, int SPLIT, int PARAB>
+__device__ __noinline__ void vol_node_fp64(const double* U, const double* Pe, const double* Ge, const double* Me,
+                                           const double* Flux, const int* es, const double* DVS, const double* DhatT,
+                                           double Lhm0, double LhpN, const Gas<double>& gas, int node, double ut[5]) {
+  constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP, N = NP - 1;
+  auto load = [&](int x, PairNode<double>& a) {
+    a.rho = Pe[x]; a.u = Pe[n3 + x]; a.v = Pe[2 * n3 + x]; a.w = Pe[3 * n3 + x]; a.pm = Pe[4 * n3 + x];
+    a.m1 = a.m2 = a.m3 = 0.;
+    a.aux = pair_aux<SPLIT, double>(a.rho, a.u, a.v, a.w, U[x * 5 + 4], a.pm, Pe[6 * n3 + x]);
+  };
+  const int ijk[3] = {node % n, (node / n) % n, node / n2};
+  double acc[5] = {0., 0., 0., 0., 0.};
+  PairNode<double> a;
+  load(node, a);
+#pragma unroll 1
+  for (int dir = 0; dir < 3; ++dir) {
+    const int step = dir == 0 ? 1 : (dir == 1 ? n : n2), i = ijk[dir], base = node - i * step;
+    const double* M = Me + (size_t)3 * dir * n3;
+#pragma unroll 1
+    for (int l = 0; l < n; ++l) {
+      const int x = base + l * step;
+      PairNode<double> b;
+      load(x, b);
+      if (l != i) {
+        double F[5];
+        split_pair_flux<SPLIT, double>(a, b, M[node] + M[x], M[n3 + node] + M[n3 + x], M[2 * n3 + node] + M[2 * n3 + x],
+                                       0., F);
+        for (int v = 0; v < 5; ++v) acc[v] = acc[v] + DVS[l + n * i] * F[v];
+      }
+      if constexpr (PARAB) {
+        double g[15], tau[6], tq[3];
+        for (int c = 0; c < 15; ++c) g[c] = c % 5 ? Ge[c * n3 + x] : 0.;
+        const double vel[3] = {b.u, b.v, b.w};
+        visc_stress(g, g + 5, g + 10, vel, gas.mu, gas.lambda, tau, tq);
+        const double m0 = M[x], m1 = M[n3 + x], m2 = M[2 * n3 + x], d = DhatT[l + n * i];
+        acc[1] = acc[1] + d * (-m0 * tau[0] - m1 * tau[3] - m2 * tau[4]);
+        acc[2] = acc[2] + d * (-m0 * tau[3] - m1 * tau[1] - m2 * tau[5]);
+        acc[3] = acc[3] + d * (-m0 * tau[4] - m1 * tau[5] - m2 * tau[2]);
+        acc[4] = acc[4] + d * (-m0 * tq[0] - m1 * tq[1] - m2 * tq[2]);
+      }
+    }
+  }
+#pragma unroll 1
+  for (int ls = 1; ls <= 6; ++ls) {
+    const int dir = ls == L_XI_MINUS || ls == L_XI_PLUS ? 0 : (ls == L_ETA_MINUS || ls == L_ETA_PLUS ? 1 : 2);
+    if (ijk[dir] != (is_minus(ls) ? 0 : N)) continue;
+    const int fa = dir == 0 ? ijk[1] : ijk[0], fb = dir == 2 ? ijk[1] : ijk[2];
+    const int side = es[2 * (ls - 1)], flip = es[2 * (ls - 1) + 1];
+    int p, q;
+    s2v2_inv(N, fa, fb, flip, ls, p, q);
+    const double Lh = is_minus(ls) ? Lhm0 : LhpN;
+    for (int v = 0; v < 5; ++v) {
+      const double f = Flux[((size_t)side * 5 + v) * n2 + p + n * q];
+      acc[v] = acc[v] + (flip == 0 ? f : -f) * Lh;
+    }
+  }
+  const double sj = Me[(size_t)9 * n3 + node];
+  for (int v = 0; v < 5; ++v) ut[v] = acc[v] * -1. * sj;
+}
+
+template <int NP, int SPLIT, int PARAB>
+__global__ void __launch_bounds__(VolFx<NP>::NT, VolFx<NP>::MINB)
+k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const double* __restrict__ Gvol,
+            const double* __restrict__ Met, const float* __restrict__ MetL, const double* __restrict__ Flux,
+            const int* __restrict__ E2S, const VolFxBasis<NP>* __restrict__ fxb, DevBasis<double> basis, double iw0,
+            Gas<double> gas, RKArgs rk, int rkmode) {
+  using C = VolFx<NP>;
+  constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP, N = NP - 1, NT = C::NT, NPT = C::NPT, DS = C::dslots(PARAB);
+  constexpr int OWN = C::OWN, TPL = C::TPL;
+  constexpr int S_RHO = 0, S_AUX = 1, S_VEL = 2, S_P = 5;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  fx64* const A = reinterpret_cast<fx64*>(smem_raw);
+  __shared__ VolFxBasis<NP> sb;
+  __shared__ unsigned mag[X_N];
+  __shared__ VolFxScale sc;
+  __shared__ int es[12];
+  const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < X_N) mag[tid] = tid < X_NMAX ? 0u : 0xffffffffu;
+  if (tid < 12) es[tid] = E2S[(size_t)e * 12 + tid];
+  for (int t = tid; t < n2; t += NT) sb.Q[t] = fxb->Q[t];
+  if (tid < n) sb.iw[tid] = fxb->iw[tid];
+  __syncthreads();
+  const double* const Pe = Pvol + (size_t)e * 7 * n3;
+  const double* const Me = Met + (size_t)e * 10 * n3;
+  const double* const Ue = U + (size_t)e * 5 * n3;
+  const double* const Ge = PARAB ? Gvol + (size_t)e * 15 * n3 : nullptr;
+
+  // ---- largest magnitudes of the element: node data, viscous stresses, face fluxes
+  double nd[NPT][6], tau[NPT][6], tq[NPT][3];
+  {
+    unsigned f[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    for (int t = tid; t < 6 * n2; t += NT) {
+      const int ls = t / n2 + 1, pq = t - (ls - 1) * n2;
+      const double* fx = Flux + (size_t)es[2 * (ls - 1)] * 5 * n2 + pq;
+      const unsigned f0 = fx_mag(fx[0]), fe = fx_mag(fx[4 * n2]);
+      const unsigned fm = max(fx_mag(fx[n2]), max(fx_mag(fx[2 * n2]), fx_mag(fx[3 * n2])));
+      const int dir = ls == L_XI_MINUS || ls == L_XI_PLUS ? 0 : (ls == L_ETA_MINUS || ls == L_ETA_PLUS ? 1 : 2);
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (d == dir) {
+          f[0][d] = max(f[0][d], f0);
+          f[1][d] = max(f[1][d], fm);
+          f[2][d] = max(f[2][d], fe);
+        }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      fx_block_max(f[0][d], &mag[X_F0 + d]);
+      fx_block_max(f[1][d], &mag[X_FM + d]);
+      fx_block_max(f[2][d], &mag[X_FE + d]);
+    }
+    unsigned m[6] = {0, 0, 0, 0, 0, 0}, rmin = 0xffffffffu, pmin = 0xffffffffu;
+#pragma unroll
+    for (int it = 0; it < NPT; ++it) {
+      const int node = tid + it * NT;
+      if (node < n3) {
+        const double* P = Pe + node;
+        nd[it][0] = P[0];
+        nd[it][2] = P[n3]; nd[it][3] = P[2 * n3]; nd[it][4] = P[3 * n3]; nd[it][5] = P[4 * n3];
+        nd[it][1] = pair_aux<SPLIT, double>(nd[it][0], nd[it][2], nd[it][3], nd[it][4], Ue[node * 5 + 4], nd[it][5],
+                                            P[6 * n3]);
+        const unsigned r = fx_mag(nd[it][0]), p = fx_mag(nd[it][5]);
+        m[X_RHO] = max(m[X_RHO], r);
+        rmin = min(rmin, r);
+        m[X_AUX] = max(m[X_AUX], fx_mag(nd[it][1]));
+        m[X_P] = max(m[X_P], p);
+        pmin = min(pmin, p);
+        const float u = fx_float(fx_mag(nd[it][2])), v = fx_float(fx_mag(nd[it][3])), w = fx_float(fx_mag(nd[it][4]));
+        m[X_U2] = max(m[X_U2], __float_as_uint(u * u + v * v + w * w));
+        if constexpr (PARAB) {
+          const double* G = Ge + node;
+          const double gx[5] = {0., G[n3], G[2 * n3], G[3 * n3], G[4 * n3]};
+          const double gy[5] = {0., G[6 * n3], G[7 * n3], G[8 * n3], G[9 * n3]};
+          const double gz[5] = {0., G[11 * n3], G[12 * n3], G[13 * n3], G[14 * n3]};
+          visc_stress(gx, gy, gz, &nd[it][2], gas.mu, gas.lambda, tau[it], tq[it]);
+#pragma unroll
+          for (int c = 0; c < 6; ++c) m[X_TAU] = max(m[X_TAU], fx_mag(tau[it][c]));
+#pragma unroll
+          for (int c = 0; c < 3; ++c) m[X_TQ] = max(m[X_TQ], fx_mag(tq[it][c]));
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < (PARAB ? 6 : 4); ++c) fx_block_max(m[c], &mag[c]);
+    fx_block_min(rmin, &mag[X_RHOMIN]);
+    fx_block_min(pmin, &mag[X_PMIN]);
+  }
+  __syncthreads();
+  if (warp == 0) vol_fx_scales<SPLIT, PARAB>(mag, MetL + (size_t)e * 3, sc, lane);
+  __syncthreads();
+  double* const Us = reinterpret_cast<double*>(smem_raw);  // Ut of the element, [node][5], at the end
+  if (sc.ok) {
+    // ---- node data to fixed point
+    {
+      const int r_rho = fx_r0(sc.s_rho), r_aux = fx_r0(sc.s_aux), r_vel = fx_r0(sc.s_vel), r_p = fx_r0(sc.s_p);
+      const int r_tau = fx_r0(sc.s_tau), r_tq = fx_r0(sc.s_tq);
+#pragma unroll
+      for (int it = 0; it < NPT; ++it) {
+        const int node = tid + it * NT;
+        if (node < n3) {
+          fx64* const a = A + vsw<NP>(node);
+          a[S_RHO * n3] = fx_from(nd[it][0], r_rho);
+          a[S_AUX * n3] = fx_from(nd[it][1], r_aux);
+          a[S_P * n3] = fx_from(nd[it][5], r_p);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) a[(S_VEL + c) * n3] = fx_from(nd[it][2 + c], r_vel);
+          FxLimb T[9];
+          if constexpr (PARAB) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) T[c] = fx_limb(fx_from(tau[it][c], r_tau));
+#pragma unroll
+            for (int c = 0; c < 3; ++c) T[6 + c] = fx_limb(fx_from(tq[it][c], r_tq));
+          }
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            fx64* const ad = a + (6 + d * DS) * n3;
+            const int r_M = fx_r0(sc.d[d].sM);
+            FxLimb M[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              const fx64 x = fx_from(Me[(3 * d + c) * n3 + node], r_M);
+              ad[c * n3] = x;
+              M[c] = fx_limb(x);
+            }
+            if constexpr (PARAB) {
+              // EvalTransformedDiffFlux3D: -M_d . (rows of tau), -M_d . tq
+              const int St = sc.d[d].St, kt = sc.d[d].kt, Sq = sc.d[d].Sq, kq = sc.d[d].kq;
+              auto row = [&](const FxLimb& a0, const FxLimb& a1, const FxLimb& a2, int S, int k) {
+                return -fx_sar(fx_unbias64(fx_dot(M[0], a0, M[1], a1, M[2], a2, S), S), k);
+              };
+              ad[3 * n3] = row(T[0], T[3], T[4], St, kt);
+              ad[4 * n3] = row(T[3], T[1], T[5], St, kt);
+              ad[5 * n3] = row(T[4], T[5], T[2], St, kt);
+              ad[6 * n3] = row(T[6], T[7], T[8], Sq, kq);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();
+
+    // ---- pairs, one direction after the other
+    const int lsub = lane / TPL, pos = lane - lsub * TPL;
+#pragma unroll 1
+    for (int dir = 0; dir < 3; ++dir) {
+      fx64* const Ad = A + (6 + dir * DS) * n3;
+      const int step = dir == 0 ? 1 : (dir == 1 ? n : n2);
+      const VolFxShift sh = sc.d[dir];
+      fx64 acc[C::TPW][OWN][5];
+      int so[C::TPW][OWN];
+#pragma unroll
+      for (int tw = 0; tw < C::TPW; ++tw) {
+        // lanes without a line compute the element's last one again and store nothing
+        const int li = min((warp + tw * C::NW) * C::LPW + lsub, n2 - 1);
+        const int base = dir == 0 ? n * li : (dir == 1 ? (li % n) + n2 * (li / n) : li);
+        // own nodes; the fixed-point data + 2^31 (see fx_sum)
+        fx64 rho[OWN], aux[OWN], pm[OWN], vel[OWN][3], M[OWN][3], fv[OWN][4];
+#pragma unroll
+        for (int o = 0; o < OWN; ++o) {
+          const int s = vsw<NP>(base + (pos + o * TPL) * step);
+          so[tw][o] = s;
+          rho[o] = A[S_RHO * n3 + s] + kFxHalf;
+          aux[o] = A[S_AUX * n3 + s] + kFxHalf;
+          pm[o] = A[S_P * n3 + s] + kFxHalf;
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            vel[o][c] = A[(S_VEL + c) * n3 + s] + kFxHalf;
+            M[o][c] = Ad[c * n3 + s] + kFxHalf;
+          }
+          if constexpr (PARAB) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) fv[o][c] = Ad[(3 + c) * n3 + s] + kFxHalf;
+          }
+#pragma unroll
+          for (int c = 0; c < 5; ++c) acc[tw][o][c] = 0;
+        }
+        struct Node { fx64 rho, aux, pm, vel[3], M[3], fv[4]; };
+        auto load = [&](int s, Node& b) {
+          b.rho = A[S_RHO * n3 + s]; b.aux = A[S_AUX * n3 + s]; b.pm = A[S_P * n3 + s];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) { b.vel[c] = A[(S_VEL + c) * n3 + s]; b.M[c] = Ad[c * n3 + s]; }
+          if constexpr (PARAB) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) b.fv[c] = Ad[(3 + c) * n3 + s];
+          }
+        };
+        // Q times 8 x the pair's fluxes (the density row 4 x), each with the bias of its last product; the
+        // bias cancels between the G a node adds and those it receives, except for the own pair
+        auto pair = [&](int o, const Node& b, const FxLimb Q, fx64 (&G)[5]) {
+          FxLimb us[3], Ms[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) { us[c] = fx_sum(vel[o][c], b.vel[c]); Ms[c] = fx_sum(M[o][c], b.M[c]); }
+          const fx64 V = fx_dot(Ms[0], us[0], Ms[1], us[1], Ms[2], us[2], sh.hV);
+          const FxLimb q = fx_unbias(fx_mul(fx_sum(rho[o], b.rho), fx_unbias(V, sh.hV), sh.hq), sh.hq);
+          const fx64 g = fx_unbias64(fx_mul(Q, q, sh.hg), sh.hg);
+          const FxLimb pq = fx_unbias(fx_mul(Q, fx_sum(pm[o], b.pm), sh.hp), sh.hp);
+          const FxLimb gm = fx_limb(fx_sar(g, sh.km)), gl = fx_limb(g), as = fx_sum(aux[o], b.aux);
+          G[0] = fx_sar(g, sh.k0);
+          if constexpr (PARAB) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) G[1 + c] = fx_dot(gm, us[c], pq, Ms[c], Q, fx_sum(fv[o][c], b.fv[c]), sh.hG);
+            const FxLimb f4 = fx_sum(fv[o][3], b.fv[3]);
+            if constexpr (SPLIT == DG_SPLIT_KG)
+              G[4] = fx_dot(gl, as, pq, fx_limb(fx_sar(fx_unbias64(V, sh.hV), sh.kv)), Q, f4, sh.hE);
+            else
+              G[4] = fx_dot(gl, as, Q, f4, sh.hE);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) G[1 + c] = fx_dot(gm, us[c], pq, Ms[c], sh.hG);
+            if constexpr (SPLIT == DG_SPLIT_KG)
+              G[4] = fx_dot(gl, as, pq, fx_limb(fx_sar(fx_unbias64(V, sh.hV), sh.kv)), sh.hE);
+            else
+              G[4] = fx_mul(gl, as, sh.hE);
+          }
+        };
+        auto get = [&](fx64 x, int from) { return (fx64)__shfl_sync(0xffffffffu, x, from); };
+        if constexpr (OWN == 1) {
+#pragma unroll
+          for (int d = 1; d <= n / 2; ++d) {
+            const int b = pos + d < n ? pos + d : pos + d - n;
+            Node B;
+            load(vsw<NP>(base + b * step), B);
+            fx64 G[5];
+            pair(0, B, sb.Q[b + n * pos], G);
+            const int from = lane + (pos >= d ? -d : n - d);  // the thread whose partner this node is
+#pragma unroll
+            for (int c = 0; c < 5; ++c) acc[tw][0][c] = fx_add(acc[tw][0][c], fx_sub(G[c], get(G[c], from)));
+          }
+        } else {
+          {  // the own pair
+            Node B;
+            load(so[tw][1], B);
+            fx64 G[5];
+            pair(0, B, sb.Q[pos + TPL + n * pos], G);
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+              const fx64 x = c == 0 ? G[c] : fx_unbias64(G[c], c == 4 ? sh.hE : sh.hG);
+              acc[tw][0][c] = fx_add(acc[tw][0][c], x);
+              acc[tw][1][c] = fx_sub(acc[tw][1][c], x);
+            }
+          }
+#pragma unroll
+          for (int s = 1; s <= (TPL - 1) / 2; ++s) {
+            const int b = pos + s < TPL ? pos + s : pos + s - TPL;
+            const int from = lane + (pos >= s ? -s : TPL - s);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              const int bx = b + x * TPL;
+              Node B;
+              load(vsw<NP>(base + bx * step), B);
+              fx64 G0[5], G1[5];
+              pair(0, B, sb.Q[bx + n * pos], G0);
+              pair(1, B, sb.Q[bx + n * (pos + TPL)], G1);
+#pragma unroll
+              for (int c = 0; c < 5; ++c) {
+                acc[tw][0][c] = fx_add(acc[tw][0][c], G0[c]);
+                acc[tw][1][c] = fx_add(acc[tw][1][c], G1[c]);
+                acc[tw][x][c] = fx_sub(acc[tw][x][c], get(fx_add(G0[c], G1[c]), from));
+              }
+            }
+          }
+          if constexpr (TPL % 2 == 0) {
+            // the thread n/4 places on: this thread's first node with its first, second with second; the
+            // threads of the line's second half take the other two pairs (first with second)
+            constexpr int s = TPL / 2;
+            const bool up = pos >= s;
+            const int b = up ? pos - s : pos + s, from = lane + (up ? -s : s);
+            const int b0 = up ? b + TPL : b, b1 = up ? b : b + TPL;
+            fx64 G0[5], G1[5];
+            {
+              Node B;
+              load(vsw<NP>(base + b0 * step), B);
+              pair(0, B, sb.Q[b0 + n * pos], G0);
+            }
+            {
+              Node B;
+              load(vsw<NP>(base + b1 * step), B);
+              pair(1, B, sb.Q[b1 + n * (pos + TPL)], G1);
+            }
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+              // what the other thread's pairs give this thread's first and second node
+              const fx64 r0 = get(up ? G1[c] : G0[c], from), r1 = get(up ? G0[c] : G1[c], from);
+              acc[tw][0][c] = fx_add(acc[tw][0][c], fx_sub(G0[c], r0));
+              acc[tw][1][c] = fx_add(acc[tw][1][c], fx_sub(G1[c], r1));
+            }
+          }
+        }
+      }
+      __syncthreads();  // the direction's metric terms and viscous fluxes are read
+#pragma unroll
+      for (int tw = 0; tw < C::TPW; ++tw) {
+        const int li = (warp + tw * C::NW) * C::LPW + lsub;
+        if (lsub < C::LPW && li < n2) {
+#pragma unroll
+          for (int o = 0; o < OWN; ++o)
+#pragma unroll
+            for (int c = 0; c < 5; ++c) Ad[c * n3 + so[tw][o]] = acc[tw][o][c];
+        }
+      }
+    }
+    __syncthreads();
+
+    // ---- face fluxes onto the end nodes of their lines (a direction's two faces share no node)
+    for (int t = tid; t < 6 * n2; t += NT) {
+      const int ls = t / n2 + 1, ab = t - (ls - 1) * n2;
+      const int a = ab % n, b = ab / n;
+      const int side = es[2 * (ls - 1)], flip = es[2 * (ls - 1) + 1];
+      int p, q;
+      s2v2_inv(N, a, b, flip, ls, p, q);
+      const double* f = Flux + (size_t)side * 5 * n2 + p + n * q;
+      const int dir = ls == L_XI_MINUS || ls == L_XI_PLUS ? 0 : (ls == L_ETA_MINUS || ls == L_ETA_PLUS ? 1 : 2);
+      fx64* const o = A + (6 + dir * DS) * n3 + vsw<NP>(face_node(n, ls, a, b, is_minus(ls) ? 0 : N));
+      const int r0 = fx_r0(sc.d[dir].t[0] + 2), rm = fx_r0(sc.d[dir].t[1] + 3), r4 = fx_r0(sc.d[dir].t[2] + 3);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        const fx64 x = fx_from(f[v * n2], v == 0 ? r0 : (v == 4 ? r4 : rm));
+        o[v * n3] += flip == 0 ? x : -x;
+      }
+    }
+    __syncthreads();
+
+    // ---- 1/w of the three directions, -1, the Jacobian
+#pragma unroll
+    for (int it = 0; it < NPT; ++it) {
+      const int node = tid + it * NT;
+      if (node < n3) {
+        const int i = node % n, j = (node / n) % n, k = node / n2;
+        const FxLimb w[3] = {sb.iw[i], sb.iw[j], sb.iw[k]};
+        const fx64* const a = A + vsw<NP>(node);
+        const double c = -iw0 * Me[9 * n3 + node];
+        const int ch = __double2hiint(c), cl = __double2loint(c);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+          const int r = v == 0 ? 0 : (v == 4 ? 2 : 1);
+          fx64 m = 0;
+          FxLimb x[3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            // to the smallest of the three directions' scales, halved for the range of the sum
+            x[d] = fx_limb(fx_sar(a[(6 + d * DS + v) * n3], min(sc.d[d].t[r] - sc.t[r] + 1, 63)));
+            m = fx_mid(x[d], w[d], m);
+          }
+          fx64 t = m >> 32;
+#pragma unroll
+          for (int d = 0; d < 3; ++d) t = fx_mad(x[d].h, w[d].h, t);
+          Us[node * 5 + v] = fx_to_double(t, m) * __hiloint2double(ch - ((sc.t[r] + (v == 0 ? 2 : 3) - 5) << 20), cl);
+        }
+      }
+    }
+  } else {
+    for (int node = tid; node < n3; node += NT) {
+      double ut[5];
+      vol_node_fp64<NP, SPLIT, PARAB>(Ue, Pe, Ge, Me, Flux, es, basis.DVS, basis.DhatT, basis.Lhm[0], basis.Lhp[N], gas,
+                                      node, ut);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) Us[node * 5 + v] = ut[v];
+    }
+  }
+  __syncthreads();
+  // output / LSERK-W2 stage, one value per thread in turn (the element's record is contiguous)
+  const size_t g0 = (size_t)e * 5 * n3;
+  for (int t = tid; t < 5 * n3; t += NT) {
+    const double val = Us[t];
+    if (rkmode == 0) {
+      rk.Ut[g0 + t] = val;
+    } else {
+      const double utmp = rk.Ut_tmp[g0 + t] * rk.mRKA + val;
+      rk.Ut_tmp[g0 + t] = utmp;
+      rk.U[g0 + t] = rk.U[g0 + t] + utmp * rk.b_dt;
+    }
+  }
+}
+
+}  // namespace gx
