@@ -156,7 +156,8 @@ int upload_fx_basis(dg_ctx* ctx) {
       }
     dd_legendre(N, x[i], P[i], dP);
   }
-  std::vector<int> h(2 * (size_t)(n * n + n), 0);
+  std::vector<int>& h = ctx->fxh;
+  h.assign(2 * (size_t)(n * n + n), 0);
   auto put = [&](int at, long long v) {
     const int l = (int)(unsigned)(unsigned long long)v;
     h[2 * at] = (int)((v - l) / (1ll << 32));
@@ -174,6 +175,40 @@ int upload_fx_basis(dg_ctx* ctx) {
   if (!ctx->fxb.alloc(h.size())) { set_error("cudaMalloc fixed-point basis"); return DG_ERR_ALLOC; }
   CUDA_TRY(cudaMemcpy(ctx->fxb.p, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice), "upload fixed-point basis");
   return DG_OK;
+}
+
+// SurfElem n of every side equals the metric terms of both elements at their face nodes (Gauss-Lobatto nodes;
+// minus faces: with the opposite sign) to the last bits (2^-51 of SurfElem)
+bool face_metrics_exact(int n, int nElems, const std::vector<double>& met, const std::vector<double>& fgeo,
+                        const std::vector<int>& e2s) {
+  const int N = n - 1, n2 = n * n, n3 = n2 * n;
+  for (size_t e = 0; e < (size_t)nElems; ++e)
+    for (int ls = 1; ls <= 6; ++ls) {
+      const int dir = ls == gx::L_XI_MINUS || ls == gx::L_XI_PLUS ? 0 : (ls == gx::L_ETA_MINUS || ls == gx::L_ETA_PLUS ? 1 : 2);
+      const bool minus = ls == gx::L_XI_MINUS || ls == gx::L_ETA_MINUS || ls == gx::L_ZETA_MINUS;
+      const size_t side = e2s[(e * 6 + ls - 1) * 2];
+      const int flip = e2s[(e * 6 + ls - 1) * 2 + 1];
+      const double sg = (minus ? -1. : 1.) * (flip == 0 ? 1. : -1.);
+      for (int b = 0; b < n; ++b)
+        for (int a = 0; a < n; ++a) {
+          // volume face coordinates -> side node (s2v2_inv)
+          int pp = a, qq = b;
+          if (ls == gx::L_XI_MINUS || ls == gx::L_ZETA_MINUS) { pp = b; qq = a; }
+          else if (ls == gx::L_ETA_PLUS) pp = N - a;
+          int p = pp, q = qq;
+          if (flip == 1) { p = qq; q = pp; }
+          else if (flip == 2) p = N - pp;
+          else if (flip == 3) { p = N - qq; q = N - pp; }
+          else if (flip == 4) q = N - qq;
+          const int l = minus ? 0 : N;
+          const int node = dir == 0 ? l + n * (a + n * b) : (dir == 1 ? a + n * (l + n * b) : a + n * (b + n * l));
+          const double* f = &fgeo[side * 10 * n2 + p + n * q];
+          const double se = f[9 * n2];
+          for (int c = 0; c < 3; ++c)
+            if (!(std::fabs(sg * se * f[c * n2] - met[(e * 10 + 3 * dir + c) * n3 + node]) <= se * 4.5e-16)) return false;
+        }
+    }
+  return true;
 }
 
 int run_rhs(dg_ctx* ctx, const double* U, gx::RKArgs rk, int rkmode, cudaStream_t st) {
@@ -564,7 +599,8 @@ int dg_ctx_create(const dg_config* cfg, dg_ctx** out) {
   int rc = upload_basis(ctx, ctx->d);
   if (rc == DG_OK && cfg->precision == DG_PRECISION_MIXED) rc = upload_basis(ctx, ctx->f);
   if (rc == DG_OK) rc = (cfg->precision == DG_PRECISION_FP64) ? T->configure_d() : T->configure_f();
-  if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64 && cfg->split_dg >= 0) rc = upload_fx_basis(ctx);
+  if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64 && cfg->node_type == DG_NODETYPE_GAUSS_LOBATTO)
+    rc = upload_fx_basis(ctx);
   if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64) rc = fx_table_for(ctx->n)->configure(ctx);
   if (rc == DG_OK && !(ctx->red.alloc(2) && ctx->bad.alloc(1) && ctx->kerr.alloc(1))) { set_error("cudaMalloc"); rc = DG_ERR_ALLOC; }
   if (rc == DG_OK && cudaMemset(ctx->kerr.p, 0, sizeof(int)) != cudaSuccess) { set_error("clear error flag"); rc = DG_ERR_CUDA; }
@@ -702,6 +738,18 @@ int dg_set_mesh(dg_ctx* ctx, int nElems, int nSides, int nBCSides, const double*
       }
       for (int d = 0; d < 3; ++d) hl[e * 3 + d] = fine ? (float)(0.5 * std::log2(big[d]) + 1e-5) : gx::kFxNoScale;
     }
+    // the fixed-point lifting: one scale for the metric terms of an element's three directions
+    bool flat = false;
+    for (size_t e = 0; e < (size_t)nElems; ++e) {
+      const float* l = &hl[e * 3];
+      const float a = std::fmin(l[0], std::fmin(l[1], l[2])), b = std::fmax(l[0], std::fmax(l[1], l[2]));
+      flat = flat || b - a > 8.f;
+    }
+    const dg_config& c = ctx->cfg;
+    const bool gl = c.node_type == DG_NODETYPE_GAUSS_LOBATTO;
+    ctx->lift_fx = c.parabolic && gl && ctx->N >= 2 && c.lifting == DG_LIFTING_BR1 && !c.do_weak_lifting &&
+                   !c.do_conservative_lifting && !flat;
+    ctx->face_exact = gl && face_metrics_exact(n, nElems, met, fgeo, he2s);
     if (!ctx->MetL.alloc(hl.size())) { set_error("cudaMalloc mesh"); return DG_ERR_ALLOC; }
     CUDA_TRY(cudaMemcpy(ctx->MetL.p, hl.data(), hl.size() * sizeof(float), cudaMemcpyHostToDevice), "upload metric scales");
   }

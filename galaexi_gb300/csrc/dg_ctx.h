@@ -123,7 +123,10 @@ struct dg_ctx {
   // FP64 form, block fixed-point kernels: log2 of the largest |M_d| of each element and direction
   // (kFxNoScale: outside the range of the scales), and the basis as limbs (VolFxBasis)
   gxc::DBuf<float> MetL;
+  bool lift_fx = false;    // fixed-point lifting: BR1, strong non-conservative, Gauss-Lobatto, no element flatter than 2^8
+  bool face_exact = false; // SurfElem n = +-M of both elements' face nodes to the last bits (affine elements)
   gxc::DBuf<int> fxb;
+  std::vector<int> fxh;    // ... and on the host
   gxc::DBuf<int> S2E;      // [side][5]: master elem, master local side, slave elem, slave local side, flip (0-based)
   gxc::DBuf<double> wq;    // 1D quadrature weights (n)
   // tangent-linear operator (R = S = Dual<1>), set up on first use
@@ -189,6 +192,8 @@ struct FxTable {
   int (*configure)(const dg_ctx*);
   // volume kernel of the split forms PI and KG (Gauss-Lobatto nodes)
   int (*volume)(dg_ctx*, const double* U, const gx::Gas<double>& gas, gx::RKArgs rk, int rkmode, cudaStream_t st);
+  // lifting kernel where ctx->lift_fx
+  void (*lift)(dg_ctx*, cudaStream_t st);
 };
 
 }  // namespace gxc

@@ -128,4 +128,48 @@ __device__ __forceinline__ void fx_block_min(unsigned v, unsigned* s) {
   if ((threadIdx.x & 31) == 0) atomicMin(s, v);
 }
 
+// ---- digits: X = h 2^30 + l with |l| < 2^30 (same sign as h or 0 <= l), |X| < 2^60.  Sums are taken digit by
+// digit (two additions, |l| < 2^31), products are a.h b.h + (a.h b.l + a.l b.h) / 2^30, in units of 2^60.
+struct FxDig {
+  int h, l;
+};
+__device__ __forceinline__ FxDig fd_split(fx64 x) { return {(int)(x >> 30), (int)x & 0x3fffffff}; }
+__device__ __forceinline__ fx64 fd_join(FxDig a) { return ((fx64)a.h << 30) + a.l; }
+__device__ __forceinline__ FxDig operator+(FxDig a, FxDig b) { return {a.h + b.h, a.l + b.l}; }
+__device__ __forceinline__ FxDig operator-(FxDig a, FxDig b) { return {a.h - b.h, a.l - b.l}; }
+struct FxDot {
+  fx64 hh, mid, ll;
+  __device__ __forceinline__ FxDot() : hh(0), mid(0), ll(0) {}
+  __device__ __forceinline__ void add(FxDig a, FxDig b) {
+    hh = fx_mad(a.h, b.h, hh);
+    mid = fx_mad(a.l, b.h, fx_mad(a.h, b.l, mid));
+    ll = fx_mad(a.l, b.l, ll);
+  }
+  // the low products' carry, before more than four of them (2^61 each) have been added
+  __device__ __forceinline__ void carry() { mid += ll >> 30; ll = 0; }
+  // the sum * 2^K in units of 2^60
+  template <int K = 0> __device__ __forceinline__ fx64 sum() const {
+    const fx64 m = mid + (ll >> 30);
+    return K == 0 ? hh + (m >> 30) : (hh << K) + (m >> (30 - K));
+  }
+};
+// x * 2^s towards zero in digits, from r0 = fx_r0(s); |x 2^s| < 2^60
+__device__ __forceinline__ FxDig fd_from(double x, int r0) {
+  const int hi = __double2hiint(x);
+  const unsigned lo = (unsigned)__double2loint(x);
+  const int eb = (hi >> 20) & 0x7ff;
+  const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+  const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, 11) << 32) | (lo << 11);
+  unsigned long long v;
+  asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(eb == 0 ? 64 : r0 - eb));
+  const int sg = (hi >> 31) | 1;
+  return {(int)(v >> 30) * sg, (int)((unsigned)v & 0x3fffffffu) * sg};
+}
+// x as a double times 2^k
+__device__ __forceinline__ double fx_scaled(fx64 x, int k) {
+  const double d = __ll2double_rn(x);
+  const int dh = __double2hiint(d);
+  return __hiloint2double((dh & 0x7ff00000) ? dh + (k << 20) : 0, __double2loint(d));
+}
+
 }  // namespace gx

@@ -211,6 +211,13 @@ void rhs_front(dg_ctx* ctx, PrecData<R>& P, const S* U, const gx::Gas<R>& gas, c
         lines = true;
       }
     }
+    if constexpr (std::is_same<R, double>::value && V0 == 1) {
+      // FP64 form, Gauss-Lobatto BR1 in strong non-conservative form: fixed point
+      if (ctx->lift_fx) {
+        GX_CAT(gx_fx_table_, GX_NP).lift(ctx, st);
+        lines = true;
+      }
+    }
     if (!lines)
       gx::k_lift<NP, R, V0><<<grid, NT, lift_smem<R>(), st>>>(P.Pvol.p, P.Met.p, P.Pf.p, P.Fgeo.p, ctx->E2S.p, b, L,
                                                               P.Gvol.p, P.Gf.p);
