@@ -196,6 +196,10 @@ struct FxTable {
   void (*lift)(dg_ctx*, cudaStream_t st);
 };
 
+// face fluxes of the connected sides in the FP64 form (dg_face_fx.cu); false: solver or central part without
+// a kernel there
+bool face_dp(const dg_ctx* ctx, const gx::Gas<double>& gas, cudaStream_t st);
+
 }  // namespace gxc
 
 #define GX_DECLARE_NP(NPV)                   \

@@ -226,11 +226,12 @@ void rhs_front(dg_ctx* ctx, PrecData<R>& P, const S* U, const gx::Gas<R>& gas, c
   if (ev) cudaEventRecord(ev[2], st);
   if (face) {
     const long long nt = (long long)(ctx->nSides - ctx->nBCSides) * NP * NP;
-    if (nt > 0) {
+    bool done = false;
+    if constexpr (std::is_same<R, double>::value) done = nt > 0 && gxc::face_dp(ctx, gas, st);
+    if (nt > 0 && !done)
       gx::k_face<R><<<(int)((nt + 127) / 128), 128, 0, st>>>(P.Uf.p, P.Pf.p, P.Gf.p, P.Fgeo.p, gas, L, NP * NP,
                                                                P.Flux.p);
-      ctx->launches++;
-    }
+    if (nt > 0) ctx->launches++;
     if (nbc > 0) {
       gx::k_bc_face<R><<<(int)((nbc + 255) / 256), 256, 0, st>>>(P.Pf.p, P.Gf.p, P.Fgeo.p, gas, L, NP * NP, P.Flux.p);
       ctx->launches++;
