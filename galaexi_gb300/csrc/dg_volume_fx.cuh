@@ -33,7 +33,7 @@ template <int NP> struct VolFx {
   static constexpr int TPL = NP / OWN;                            // threads per line
   static constexpr int LPW = 32 / TPL;                            // lines per warp
   static constexpr int TPD = (NP * NP + LPW - 1) / LPW;           // warp tasks per direction
-  static constexpr int TPW = OWN == 1 && TPD > 1 ? 2 : 1;         // tasks of one warp per direction
+  static constexpr int TPW = (OWN == 1 && TPD > 1) || TPD > 16 ? 2 : 1;         // tasks of one warp per direction
   static constexpr int NW = (TPD + TPW - 1) / TPW, NT = 32 * NW;  // warps and threads of a block
   static constexpr int NPT = (NP * NP * NP + NT - 1) / NT;        // nodes per thread
   // blocks per SM for 128 registers per thread (512 threads), where shared memory holds them
@@ -247,7 +247,8 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
   const double* const Ge = PARAB ? Gvol + (size_t)e * 15 * n3 : nullptr;
 
   // ---- largest magnitudes of the element: node data, viscous stresses, face fluxes
-  double nd[NPT][6], tau[NPT][6], tq[NPT][3];
+  // (the values wait in the node's own shared-memory slots as FP64 for the scales: slots 0-5 the node data,
+  // 6-14 the stresses)
   {
     unsigned f[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
     for (int t = tid; t < 6 * n2; t += NT) {
@@ -271,33 +272,40 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
       fx_block_max(f[2][d], &mag[X_FE + d]);
     }
     unsigned m[6] = {0, 0, 0, 0, 0, 0}, rmin = 0xffffffffu, pmin = 0xffffffffu;
+#pragma unroll 1
+    for (int node = tid; node < n3; node += NT) {
+      const double* P = Pe + node;
+      fx64* const a = A + vsw<NP>(node);
+      const double rho = P[0], vel[3] = {P[n3], P[2 * n3], P[3 * n3]}, p = P[4 * n3];
+      const double aux = pair_aux<SPLIT, double>(rho, vel[0], vel[1], vel[2], Ue[node * 5 + 4], p, P[6 * n3]);
+      a[S_RHO * n3] = __double_as_longlong(rho);
+      a[S_AUX * n3] = __double_as_longlong(aux);
+      a[S_P * n3] = __double_as_longlong(p);
 #pragma unroll
-    for (int it = 0; it < NPT; ++it) {
-      const int node = tid + it * NT;
-      if (node < n3) {
-        const double* P = Pe + node;
-        nd[it][0] = P[0];
-        nd[it][2] = P[n3]; nd[it][3] = P[2 * n3]; nd[it][4] = P[3 * n3]; nd[it][5] = P[4 * n3];
-        nd[it][1] = pair_aux<SPLIT, double>(nd[it][0], nd[it][2], nd[it][3], nd[it][4], Ue[node * 5 + 4], nd[it][5],
-                                            P[6 * n3]);
-        const unsigned r = fx_mag(nd[it][0]), p = fx_mag(nd[it][5]);
-        m[X_RHO] = max(m[X_RHO], r);
-        rmin = min(rmin, r);
-        m[X_AUX] = max(m[X_AUX], fx_mag(nd[it][1]));
-        m[X_P] = max(m[X_P], p);
-        pmin = min(pmin, p);
-        const float u = fx_float(fx_mag(nd[it][2])), v = fx_float(fx_mag(nd[it][3])), w = fx_float(fx_mag(nd[it][4]));
-        m[X_U2] = max(m[X_U2], __float_as_uint(u * u + v * v + w * w));
-        if constexpr (PARAB) {
-          const double* G = Ge + node;
-          const double gx[5] = {0., G[n3], G[2 * n3], G[3 * n3], G[4 * n3]};
-          const double gy[5] = {0., G[6 * n3], G[7 * n3], G[8 * n3], G[9 * n3]};
-          const double gz[5] = {0., G[11 * n3], G[12 * n3], G[13 * n3], G[14 * n3]};
-          visc_stress(gx, gy, gz, &nd[it][2], gas.mu, gas.lambda, tau[it], tq[it]);
+      for (int c = 0; c < 3; ++c) a[(S_VEL + c) * n3] = __double_as_longlong(vel[c]);
+      m[X_RHO] = max(m[X_RHO], fx_mag(rho));
+      rmin = min(rmin, fx_mag(rho));
+      m[X_AUX] = max(m[X_AUX], fx_mag(aux));
+      m[X_P] = max(m[X_P], fx_mag(p));
+      pmin = min(pmin, fx_mag(p));
+      const float u = fx_float(fx_mag(vel[0])), v = fx_float(fx_mag(vel[1])), w = fx_float(fx_mag(vel[2]));
+      m[X_U2] = max(m[X_U2], __float_as_uint(u * u + v * v + w * w));
+      if constexpr (PARAB) {
+        const double* G = Ge + node;
+        const double gx[5] = {0., G[n3], G[2 * n3], G[3 * n3], G[4 * n3]};
+        const double gy[5] = {0., G[6 * n3], G[7 * n3], G[8 * n3], G[9 * n3]};
+        const double gz[5] = {0., G[11 * n3], G[12 * n3], G[13 * n3], G[14 * n3]};
+        double tau[6], tq[3];
+        visc_stress(gx, gy, gz, vel, gas.mu, gas.lambda, tau, tq);
 #pragma unroll
-          for (int c = 0; c < 6; ++c) m[X_TAU] = max(m[X_TAU], fx_mag(tau[it][c]));
+        for (int c = 0; c < 6; ++c) {
+          m[X_TAU] = max(m[X_TAU], fx_mag(tau[c]));
+          a[(6 + c) * n3] = __double_as_longlong(tau[c]);
+        }
 #pragma unroll
-          for (int c = 0; c < 3; ++c) m[X_TQ] = max(m[X_TQ], fx_mag(tq[it][c]));
+        for (int c = 0; c < 3; ++c) {
+          m[X_TQ] = max(m[X_TQ], fx_mag(tq[c]));
+          a[(12 + c) * n3] = __double_as_longlong(tq[c]);
         }
       }
     }
@@ -315,45 +323,43 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
     {
       const int r_rho = fx_r0(sc.s_rho), r_aux = fx_r0(sc.s_aux), r_vel = fx_r0(sc.s_vel), r_p = fx_r0(sc.s_p);
       const int r_tau = fx_r0(sc.s_tau), r_tq = fx_r0(sc.s_tq);
+#pragma unroll 1
+      for (int node = tid; node < n3; node += NT) {
+        fx64* const a = A + vsw<NP>(node);
+        auto raw = [&](int slot) { return __longlong_as_double(a[slot * n3]); };
+        FxLimb T[9];
+        if constexpr (PARAB) {
 #pragma unroll
-      for (int it = 0; it < NPT; ++it) {
-        const int node = tid + it * NT;
-        if (node < n3) {
-          fx64* const a = A + vsw<NP>(node);
-          a[S_RHO * n3] = fx_from(nd[it][0], r_rho);
-          a[S_AUX * n3] = fx_from(nd[it][1], r_aux);
-          a[S_P * n3] = fx_from(nd[it][5], r_p);
+          for (int c = 0; c < 6; ++c) T[c] = fx_limb(fx_from(raw(6 + c), r_tau));
 #pragma unroll
-          for (int c = 0; c < 3; ++c) a[(S_VEL + c) * n3] = fx_from(nd[it][2 + c], r_vel);
-          FxLimb T[9];
-          if constexpr (PARAB) {
+          for (int c = 0; c < 3; ++c) T[6 + c] = fx_limb(fx_from(raw(12 + c), r_tq));
+        }
+        a[S_RHO * n3] = fx_from(raw(S_RHO), r_rho);
+        a[S_AUX * n3] = fx_from(raw(S_AUX), r_aux);
+        a[S_P * n3] = fx_from(raw(S_P), r_p);
 #pragma unroll
-            for (int c = 0; c < 6; ++c) T[c] = fx_limb(fx_from(tau[it][c], r_tau));
+        for (int c = 0; c < 3; ++c) a[(S_VEL + c) * n3] = fx_from(raw(S_VEL + c), r_vel);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) T[6 + c] = fx_limb(fx_from(tq[it][c], r_tq));
+        for (int d = 0; d < 3; ++d) {
+          fx64* const ad = a + (6 + d * DS) * n3;
+          const int r_M = fx_r0(sc.d[d].sM);
+          FxLimb M[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const fx64 x = fx_from(Me[(3 * d + c) * n3 + node], r_M);
+            ad[c * n3] = x;
+            M[c] = fx_limb(x);
           }
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            fx64* const ad = a + (6 + d * DS) * n3;
-            const int r_M = fx_r0(sc.d[d].sM);
-            FxLimb M[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              const fx64 x = fx_from(Me[(3 * d + c) * n3 + node], r_M);
-              ad[c * n3] = x;
-              M[c] = fx_limb(x);
-            }
-            if constexpr (PARAB) {
-              // EvalTransformedDiffFlux3D: -M_d . (rows of tau), -M_d . tq
-              const int St = sc.d[d].St, kt = sc.d[d].kt, Sq = sc.d[d].Sq, kq = sc.d[d].kq;
-              auto row = [&](const FxLimb& a0, const FxLimb& a1, const FxLimb& a2, int S, int k) {
-                return -fx_sar(fx_unbias64(fx_dot(M[0], a0, M[1], a1, M[2], a2, S), S), k);
-              };
-              ad[3 * n3] = row(T[0], T[3], T[4], St, kt);
-              ad[4 * n3] = row(T[3], T[1], T[5], St, kt);
-              ad[5 * n3] = row(T[4], T[5], T[2], St, kt);
-              ad[6 * n3] = row(T[6], T[7], T[8], Sq, kq);
-            }
+          if constexpr (PARAB) {
+            // EvalTransformedDiffFlux3D: -M_d . (rows of tau), -M_d . tq
+            const int St = sc.d[d].St, kt = sc.d[d].kt, Sq = sc.d[d].Sq, kq = sc.d[d].kq;
+            auto row = [&](const FxLimb& a0, const FxLimb& a1, const FxLimb& a2, int S, int k) {
+              return -fx_sar(fx_unbias64(fx_dot(M[0], a0, M[1], a1, M[2], a2, S), S), k);
+            };
+            ad[3 * n3] = row(T[0], T[3], T[4], St, kt);
+            ad[4 * n3] = row(T[3], T[1], T[5], St, kt);
+            ad[5 * n3] = row(T[4], T[5], T[2], St, kt);
+            ad[6 * n3] = row(T[6], T[7], T[8], Sq, kq);
           }
         }
       }
@@ -375,7 +381,7 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
         const int li = min((warp + tw * C::NW) * C::LPW + lsub, n2 - 1);
         const int base = dir == 0 ? n * li : (dir == 1 ? (li % n) + n2 * (li / n) : li);
         // own nodes; the fixed-point data + 2^31 (see fx_sum)
-        fx64 rho[OWN], aux[OWN], pm[OWN], vel[OWN][3], M[OWN][3], fv[OWN][4];
+        fx64 rho[OWN], aux[OWN], pm[OWN], vel[OWN][3], M[OWN][3];
 #pragma unroll
         for (int o = 0; o < OWN; ++o) {
           const int s = vsw<NP>(base + (pos + o * TPL) * step);
@@ -388,26 +394,21 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
             vel[o][c] = A[(S_VEL + c) * n3 + s] + kFxHalf;
             M[o][c] = Ad[c * n3 + s] + kFxHalf;
           }
-          if constexpr (PARAB) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) fv[o][c] = Ad[(3 + c) * n3 + s] + kFxHalf;
-          }
 #pragma unroll
           for (int c = 0; c < 5; ++c) acc[tw][o][c] = 0;
         }
-        struct Node { fx64 rho, aux, pm, vel[3], M[3], fv[4]; };
+        struct Node { fx64 rho, aux, pm, vel[3], M[3]; int s; };
         auto load = [&](int s, Node& b) {
           b.rho = A[S_RHO * n3 + s]; b.aux = A[S_AUX * n3 + s]; b.pm = A[S_P * n3 + s];
 #pragma unroll
           for (int c = 0; c < 3; ++c) { b.vel[c] = A[(S_VEL + c) * n3 + s]; b.M[c] = Ad[c * n3 + s]; }
-          if constexpr (PARAB) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b.fv[c] = Ad[(3 + c) * n3 + s];
-          }
+          b.s = s;
         };
         // Q times 8 x the pair's fluxes (the density row 4 x), each with the bias of its last product; the
         // bias cancels between the G a node adds and those it receives, except for the own pair
         auto pair = [&](int o, const Node& b, const FxLimb Q, fx64 (&G)[5]) {
+          // the viscous fluxes of both nodes are read here: held as well, they would not leave enough registers
+          auto fvs = [&](int c) { return fx_limb(Ad[(3 + c) * n3 + so[tw][o]] + Ad[(3 + c) * n3 + b.s]); };
           FxLimb us[3], Ms[3];
 #pragma unroll
           for (int c = 0; c < 3; ++c) { us[c] = fx_sum(vel[o][c], b.vel[c]); Ms[c] = fx_sum(M[o][c], b.M[c]); }
@@ -419,8 +420,8 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
           G[0] = fx_sar(g, sh.k0);
           if constexpr (PARAB) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) G[1 + c] = fx_dot(gm, us[c], pq, Ms[c], Q, fx_sum(fv[o][c], b.fv[c]), sh.hG);
-            const FxLimb f4 = fx_sum(fv[o][3], b.fv[3]);
+            for (int c = 0; c < 3; ++c) G[1 + c] = fx_dot(gm, us[c], pq, Ms[c], Q, fvs(c), sh.hG);
+            const FxLimb f4 = fvs(3);
             if constexpr (SPLIT == DG_SPLIT_KG)
               G[4] = fx_dot(gl, as, pq, fx_limb(fx_sar(fx_unbias64(V, sh.hV), sh.kv)), Q, f4, sh.hE);
             else
