@@ -99,65 +99,14 @@ int upload_basis(dg_ctx* ctx, gxc::PrecData<R>& P) {
   return DG_OK;
 }
 
-// double-double numbers (Dekker's and Knuth's error-free sum and product): the limbs of the fixed-point
-// basis need 62 bits, on every host
-struct DD {
-  double h, l;
-};
-DD dd_add(DD a, DD b) {
-  const double s = a.h + b.h, t = s - a.h;
-  const double e = (a.h - (s - t)) + (b.h - t) + a.l + b.l;
-  const double h = s + e;
-  return {h, e - (h - s)};
-}
-DD dd_mul(DD a, DD b) {
-  const double p = a.h * b.h;
-  const double e = std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
-  const double h = p + e;
-  return {h, e - (h - p)};
-}
-DD dd_neg(DD a) { return {-a.h, -a.l}; }
-DD dd_inv(DD a) {
-  const double x = 1. / a.h;
-  const DD r = dd_add({1., 0.}, dd_neg(dd_mul(a, {x, 0.})));
-  return dd_add({x, 0.}, {x * (r.h + r.l), 0.});
-}
-long long dd_fixed(DD a, int bits) { return std::llrint(std::ldexp(a.h, bits)) + std::llrint(std::ldexp(a.l, bits)); }
-// P_N and P_N' at x by the three-term recurrence
-void dd_legendre(int N, DD x, DD& P, DD& dP) {
-  DD p0{1., 0.}, p1 = x, d0{0., 0.}, d1{1., 0.};
-  for (int k = 2; k <= N; ++k) {
-    const DD a = dd_mul({2. * k - 1., 0.}, dd_inv({(double)k, 0.})), b = dd_mul({k - 1., 0.}, dd_inv({(double)k, 0.}));
-    const DD p2 = dd_add(dd_mul(a, dd_mul(x, p1)), dd_neg(dd_mul(b, p0)));
-    const DD d2 = dd_add(d0, dd_mul({2. * k - 1., 0.}, p1));
-    p0 = p1; p1 = p2; d0 = d1; d1 = d2;
-  }
-  P = p1; dP = d1;
-}
-
-// the basis of the fixed-point volume kernel (VolFxBasis) on Gauss-Lobatto nodes: Q(i,l) = w_i l_l'(x_i)
-// = 2 / (N (N+1) P_N(x_i) P_N(x_l) (x_i - x_l)) for i != l, times 2^62, and w_0/w_i = P_N(x_i)^2, times 2^60.
-// The nodes (zeros of P_N') are refined from the FP64 ones: with rounded FP64 matrices the antisymmetry
-// and the row sums of Q would only hold to 1e-15.
+// the basis of the fixed-point kernels in double-double, and the volume kernel's limbs on the device (VolFxBasis,
+// Gauss-Lobatto nodes): Q(i,l) = w_i D(i,l) 2^62, w_0/w_i 2^60.  With rounded FP64 matrices the antisymmetry and
+// the row sums of Q would only hold to 1e-15.
 int upload_fx_basis(dg_ctx* ctx) {
-  const int n = ctx->n, N = ctx->N;
-  std::vector<DD> x(n), P(n);
-  for (int i = 0; i < n; ++i) {
-    DD dP;
-    x[i] = {ctx->B.x[i], 0.};
-    if (i == 0 || i == N) x[i] = {i == 0 ? -1. : 1., 0.};
-    else
-      for (int it = 0; it < 3; ++it) {
-        // Newton on P_N': (1 - x^2) P_N'' = 2 x P_N' - N (N+1) P_N
-        dd_legendre(N, x[i], P[i], dP);
-        const DD q = dd_add({1., 0.}, dd_neg(dd_mul(x[i], x[i])));
-        const DD d2 = dd_mul(dd_add(dd_mul({2., 0.}, dd_mul(x[i], dP)), dd_neg(dd_mul({N * (N + 1.), 0.}, P[i]))), dd_inv(q));
-        x[i] = dd_add(x[i], dd_neg(dd_mul(dP, dd_inv(d2))));
-      }
-    dd_legendre(N, x[i], P[i], dP);
-  }
-  std::vector<int>& h = ctx->fxh;
-  h.assign(2 * (size_t)(n * n + n), 0);
+  const int n = ctx->n;
+  gxh::basis_dd(ctx->N, ctx->cfg.node_type, ctx->B.x, ctx->fxB);
+  if (ctx->cfg.node_type != DG_NODETYPE_GAUSS_LOBATTO) return DG_OK;
+  std::vector<int> h(2 * (size_t)(n * n + n), 0);
   auto put = [&](int at, long long v) {
     const int l = (int)(unsigned)(unsigned long long)v;
     h[2 * at] = (int)((v - l) / (1ll << 32));
@@ -165,12 +114,11 @@ int upload_fx_basis(dg_ctx* ctx) {
   };
   for (int i = 0; i < n; ++i) {
     for (int l = i + 1; l < n; ++l) {
-      const DD d = dd_mul(dd_mul(P[i], P[l]), dd_add(x[i], dd_neg(x[l])));
-      const long long q = dd_fixed(dd_mul({2., 0.}, dd_inv(dd_mul({N * (N + 1.), 0.}, d))), 62);
+      const long long q = gxh::dd_fixed(gxh::dd_mul(ctx->fxB.w[i], ctx->fxB.D[i * n + l]), 62);
       put(l + n * i, q);
       put(i + n * l, -q);
     }
-    put(n * n + i, dd_fixed(dd_mul(P[i], P[i]), 60));
+    put(n * n + i, gxh::dd_fixed(gxh::dd_mul(ctx->fxB.w[0], gxh::dd_inv(ctx->fxB.w[i])), 60));
   }
   if (!ctx->fxb.alloc(h.size())) { set_error("cudaMalloc fixed-point basis"); return DG_ERR_ALLOC; }
   CUDA_TRY(cudaMemcpy(ctx->fxb.p, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice), "upload fixed-point basis");
@@ -599,8 +547,7 @@ int dg_ctx_create(const dg_config* cfg, dg_ctx** out) {
   int rc = upload_basis(ctx, ctx->d);
   if (rc == DG_OK && cfg->precision == DG_PRECISION_MIXED) rc = upload_basis(ctx, ctx->f);
   if (rc == DG_OK) rc = (cfg->precision == DG_PRECISION_FP64) ? T->configure_d() : T->configure_f();
-  if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64 && cfg->node_type == DG_NODETYPE_GAUSS_LOBATTO)
-    rc = upload_fx_basis(ctx);
+  if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64) rc = upload_fx_basis(ctx);
   if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64) rc = fx_table_for(ctx->n)->configure(ctx);
   if (rc == DG_OK && !(ctx->red.alloc(2) && ctx->bad.alloc(1) && ctx->kerr.alloc(1))) { set_error("cudaMalloc"); rc = DG_ERR_ALLOC; }
   if (rc == DG_OK && cudaMemset(ctx->kerr.p, 0, sizeof(int)) != cudaSuccess) { set_error("clear error flag"); rc = DG_ERR_CUDA; }
@@ -715,33 +662,36 @@ int dg_set_mesh(dg_ctx* ctx, int nElems, int nSides, int nBCSides, const double*
   CUDA_TRY(cudaMemcpy(ctx->E2S.p, he2s.data(), he2s.size() * sizeof(int), cudaMemcpyHostToDevice), "upload E2S");
   ctx->MetL.release();
   if (ctx->cfg.precision == DG_PRECISION_FP64) {
-    // log2 of each element's largest |M_d| (2-norm), rounded up, for the fixed-point scales
-    std::vector<float> hl((size_t)nElems * 3);
+    // log2 of each element's largest |M_d| (2-norm) and |M_d,c|, rounded up, for the fixed-point scales
+    std::vector<float> hl((size_t)nElems * 12);
     for (size_t e = 0; e < (size_t)nElems; ++e) {
       const double* m = &met[e * 10 * n3];
       bool fine = true;
-      double big[3];
+      double big[12] = {0.};
       for (int d = 0; d < 3; ++d) {
-        double q = 0.;
         for (int t = 0; t < n3; ++t) {
-          const double a = m[(3 * d) * n3 + t], b = m[(3 * d + 1) * n3 + t], c = m[(3 * d + 2) * n3 + t];
-          const double s = a * a + b * b + c * c;
+          double s = 0.;
+          for (int c = 0; c < 3; ++c) {
+            const double a = m[(3 * d + c) * n3 + t] * m[(3 * d + c) * n3 + t];
+            s += a;
+            big[3 + 3 * d + c] = a > big[3 + 3 * d + c] ? a : big[3 + 3 * d + c];
+          }
           if (!(s < 1e90)) fine = false;
-          q = s > q ? s : q;
+          big[d] = s > big[d] ? s : big[d];
         }
-        big[d] = q;
-        if (!(q > 1e-90)) fine = false;
+        if (!(big[d] > 1e-90)) fine = false;
       }
       for (int t = 0; t < n3; ++t) {
         const double sj = std::fabs(m[9 * n3 + t]);
         if (!(sj > 1e-45 && sj < 1e45)) fine = false;
       }
-      for (int d = 0; d < 3; ++d) hl[e * 3 + d] = fine ? (float)(0.5 * std::log2(big[d]) + 1e-5) : gx::kFxNoScale;
+      for (int c = 0; c < 12; ++c)
+        hl[e * 12 + c] = !fine ? gx::kFxNoScale : (big[c] > 1e-90 ? (float)(0.5 * std::log2(big[c]) + 1e-5) : -150.f);
     }
     // the fixed-point lifting: one scale for the metric terms of an element's three directions
     bool flat = false;
     for (size_t e = 0; e < (size_t)nElems; ++e) {
-      const float* l = &hl[e * 3];
+      const float* l = &hl[e * 12];
       const float a = std::fmin(l[0], std::fmin(l[1], l[2])), b = std::fmax(l[0], std::fmax(l[1], l[2]));
       flat = flat || b - a > 8.f;
     }

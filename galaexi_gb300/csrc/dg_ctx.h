@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../../include/galaexi_gb300.h"
+#include "dg_dd.h"
 #include "dg_host.h"
 #include "dg_kernels.cuh"
 #include "dg_adjoint.cuh"
@@ -120,13 +121,14 @@ struct dg_ctx {
   long long launches = 0;
   int lines_grid = 0;      // blocks of the persistent line volume kernel (SMs x resident blocks), on first use
   int prolong_grid = 0;    // blocks of the persistent prolongation kernel of the mixed form, on first use
-  // FP64 form, block fixed-point kernels: log2 of the largest |M_d| of each element and direction
+  // FP64 form, block fixed-point kernels: log2 of the largest |M_d| (3) and |M_d,c| (9) of each element
   // (kFxNoScale: outside the range of the scales), and the basis as limbs (VolFxBasis)
   gxc::DBuf<float> MetL;
   bool lift_fx = false;    // fixed-point lifting: BR1, strong non-conservative, Gauss-Lobatto, no element flatter than 2^8
   bool face_exact = false; // SurfElem n = +-M of both elements' face nodes to the last bits (affine elements)
   gxc::DBuf<int> fxb;
-  std::vector<int> fxh;    // ... and on the host
+  gxh::BasisDD fxB;        // the basis in double-double (FP64 form)
+  std::vector<unsigned char> fx_lift, fx_weak;  // LiftFxBasis, VolWfxBasis, on first use
   gxc::DBuf<int> S2E;      // [side][5]: master elem, master local side, slave elem, slave local side, flip (0-based)
   gxc::DBuf<double> wq;    // 1D quadrature weights (n)
   // tangent-linear operator (R = S = Dual<1>), set up on first use
@@ -190,7 +192,7 @@ struct NPTable {
 // the fixed-point kernels of the FP64 form, in translation units of their own (dg_fx<NP>.cu)
 struct FxTable {
   int (*configure)(const dg_ctx*);
-  // volume kernel of the split forms PI and KG (Gauss-Lobatto nodes)
+  // volume kernel of the weak form and of the split forms PI and KG (Gauss-Lobatto nodes)
   int (*volume)(dg_ctx*, const double* U, const gx::Gas<double>& gas, gx::RKArgs rk, int rkmode, cudaStream_t st);
   // lifting kernel where ctx->lift_fx
   void (*lift)(dg_ctx*, cudaStream_t st);

@@ -3,10 +3,13 @@
 // the compiler laid the FP64 kernels of dg_np<NP>.cu out differently (prolongation at N = 5 up to 19% slower).
 #pragma once
 #include <cmath>
+#include <cstring>
+#include <vector>
 
 #include "dg_ctx.h"
 #include "dg_lift_fx.cuh"
 #include "dg_volume_fx.cuh"
+#include "dg_volume_wfx.cuh"
 
 #ifndef GX_NP
 #error "define GX_NP before including dg_fx_np.cuh"
@@ -32,6 +35,79 @@ int smem_attr(K kern, size_t bytes, const char* what) {
   return DG_OK;
 }
 
+// the exponent e with |x| < 2^e for all entries of a matrix
+int exponent(const std::vector<gxh::DD>& a) {
+  double big = 0.;
+  for (const gxh::DD& x : a) big = std::fabs(x.h) > big ? std::fabs(x.h) : big;
+  int ex = 0;
+  std::frexp(big * 1.01, &ex);
+  return ex;
+}
+gx::FxDig digits(long long x) { return gx::FxDig{(int)(x >> 30), (int)(x & 0x3fffffff)}; }
+gx::FxLimb limbs(long long x) {
+  const int l = (int)(unsigned)(unsigned long long)x;
+  return gx::FxLimb{(int)((x - l) / (1ll << 32)), l};
+}
+
+// a basis struct of a kernel, built once per context and kept there as bytes
+template <typename B, typename F>
+const B& kept(std::vector<unsigned char>& store, F build) {
+  if (store.size() != sizeof(B)) {
+    store.resize(sizeof(B));
+    B b;
+    std::memset(&b, 0, sizeof(B));
+    build(b);
+    std::memcpy(store.data(), &b, sizeof(B));
+  }
+  return *reinterpret_cast<const B*>(store.data());
+}
+
+// D_hat(i,l) = -w_l/w_i D(l,i) and L_hat(i) = L(i)/w_i in even and odd parts (VolWfxBasis).  A constant flux and
+// its face fluxes cancel exactly: the diagonal even entry is what the others leave
+void weak_basis(const dg_ctx* ctx, gx::VolWfxBasis<NP>& wb) {
+  constexpr int N = NP - 1, H = gx::VolWfxBasis<NP>::H, HE = gx::VolWfxBasis<NP>::HE;
+  const gxh::BasisDD& B = ctx->fxB;
+  std::vector<gxh::DD> Dh(NP * NP), Lh(NP), all;
+  for (int i = 0; i < NP; ++i) {
+    const gxh::DD iw = gxh::dd_inv(B.w[i]);
+    for (int l = 0; l < NP; ++l) Dh[i * NP + l] = gxh::dd_neg(gxh::dd_mul(gxh::dd_mul(B.w[l], iw), B.D[l * NP + i]));
+    Lh[i] = gxh::dd_mul(B.Lp[i], iw);
+  }
+  all = Dh;
+  all.insert(all.end(), Lh.begin(), Lh.end());
+  wb.sD = 60 - exponent(all);
+  auto half = [](gxh::DD a) { return gxh::dd_mul(a, gxh::dd_num(0.5)); };
+  auto at = [&](int i, int l) { return Dh[i * NP + l]; };
+  for (int i = 0; i < HE; ++i) {
+    // L_hat_plus(i) = Lh[i], L_hat_minus(i) = Lh[N-i]
+    const long long le = gxh::dd_fixed(half(gxh::dd_add(Lh[i], Lh[N - i])), wb.sD);
+    const long long lo = gxh::dd_fixed(half(gxh::dd_sub(Lh[i], Lh[N - i])), wb.sD);
+    wb.le[i] = limbs(le);
+    long long rest = i < H ? lo : 0;
+    if (i < H) wb.lo[i] = limbs(lo);
+    for (int l = 0; l < HE; ++l) {
+      if (i < H && l != i) {
+        const long long ev = l < H ? gxh::dd_fixed(half(gxh::dd_add(at(i, l), at(i, N - l))), wb.sD)
+                                   : gxh::dd_fixed(at(i, l), wb.sD - 1) * 2;
+        rest += l < H ? ev : ev / 2;
+        wb.even[i][l] = limbs(ev);
+      }
+      if (l < H) wb.odd[i][l] = limbs(gxh::dd_fixed(i < H ? half(gxh::dd_sub(at(i, l), at(i, N - l))) : at(i, l), wb.sD));
+    }
+    if (i < H) wb.even[i][i] = limbs(-rest);
+  }
+}
+
+int volume_weak(dg_ctx* ctx, const double* U, const gx::Gas<double>& gas, gx::RKArgs rk, int rkmode, cudaStream_t st) {
+  const gxc::PrecData<double>& P = ctx->d;
+  const auto& wb = kept<gx::VolWfxBasis<NP>>(ctx->fx_weak, [&](gx::VolWfxBasis<NP>& b) { weak_basis(ctx, b); });
+  auto kern = ctx->cfg.parabolic ? gx::k_volume_wfx<NP, 1> : gx::k_volume_wfx<NP, 0>;
+  kern<<<ctx->nElems, gx::VolWfx<NP>::NT, gx::VolWfx<NP>::smem, st>>>(
+      U, P.Pvol.p, P.Gvol.p, P.Met.p, ctx->MetL.p, P.Flux.p, ctx->E2S.p, wb, gxc::dev_basis(P, NP),
+      ctx->cfg.node_type == DG_NODETYPE_GAUSS ? 1 : 0, gas, rk, rkmode);
+  return DG_OK;
+}
+
 template <int SPL>
 int volume_spl(dg_ctx* ctx, const double* U, const gx::Gas<double>& gas, gx::RKArgs rk, int rkmode, cudaStream_t st) {
   const gxc::PrecData<double>& P = ctx->d;
@@ -43,6 +119,9 @@ int volume_spl(dg_ctx* ctx, const double* U, const gx::Gas<double>& gas, gx::RKA
 }
 
 int volume(dg_ctx* ctx, const double* U, const gx::Gas<double>& gas, gx::RKArgs rk, int rkmode, cudaStream_t st) {
+  if (ctx->cfg.split_dg == DG_SPLIT_NONE) {
+    if constexpr (NP >= 4) return volume_weak(ctx, U, gas, rk, rkmode, st);
+  }
   if constexpr (NP >= 3)
     return ctx->cfg.split_dg == DG_SPLIT_KG ? volume_spl<DG_SPLIT_KG>(ctx, U, gas, rk, rkmode, st)
                                             : volume_spl<DG_SPLIT_PI>(ctx, U, gas, rk, rkmode, st);
@@ -56,47 +135,35 @@ int configure_spl() {
   return rc ? rc : smem_attr(gx::k_volume_fx<NP, SPL, 1>, gx::VolFx<NP>::smem(1), "k_volume_fx attributes");
 }
 
-// D of the Gauss-Lobatto nodes in even and odd parts (LiftFxBasis), from the basis limbs Q(i,l) 2^62 and
-// w_0/w_i 2^60 of the context: D(i,l) = Q(i,l) / w_i = Q(i,l) (w_0/w_i) N(N+1)/2 off the diagonal, 0 on it but
-// -+N(N+1)/4 at the ends
+// D in even and odd parts (LiftFxBasis).  The even parts of a row times (x_l + x_(N-l)) vanish exactly for a
+// constant: the diagonal entry is what the others leave
 void lift_basis(const dg_ctx* ctx, gx::LiftFxBasis<NP>& lb) {
   constexpr int N = NP - 1, H = gx::LiftFxBasis<NP>::H, HE = gx::LiftFxBasis<NP>::HE;
-  auto limb = [&](int at) { return (long long)ctx->fxh[2 * at] * (1ll << 32) + ctx->fxh[2 * at + 1]; };
-  double big = 0.;
-  for (int i = 0; i < NP; ++i)
-    for (int l = 0; l < NP; ++l) big = std::fabs(ctx->B.D[i + NP * l]) > big ? std::fabs(ctx->B.D[i + NP * l]) : big;
-  int ex = 0;
-  std::frexp(big * 1.01, &ex);
-  lb.sD = 58 - ex;
-  auto D = [&](int i, int l) -> long long {  // D(i,l) 2^sD
-    if (i == l) return i == 0 || i == N ? (i == 0 ? -1 : 1) * (long long)(((__int128)(N * (N + 1)) << lb.sD) / 4) : 0;
-    const __int128 p = (__int128)limb(l + NP * i) * limb(NP * NP + i) / ((__int128)1 << 60);  // Q w_0/w_i 2^62
-    return (long long)((p * (N * (N + 1) / 2)) / ((__int128)1 << (62 - lb.sD)));
-  };
-  auto dig = [](long long x) { return gx::FxDig{(int)(x >> 30), (int)(x & 0x3fffffff)}; };
+  const std::vector<gxh::DD>& D = ctx->fxB.D;
+  lb.sD = 58 - exponent(D);
+  auto at = [&](int i, int l) { return D[i * NP + l]; };
+  auto half = [](gxh::DD a) { return gxh::dd_mul(a, gxh::dd_num(0.5)); };
   for (int i = 0; i < HE; ++i) {
-    // the even parts of a row times (x_l + x_(N-l)) vanish exactly for a constant: the diagonal entry is what
-    // the others leave
     long long rest = 0;
     for (int l = 0; l < HE; ++l) {
-      long long ev = 0;
       if (i < H && l != i) {
-        ev = l < H ? (D(i, l) + D(i, N - l)) / 2 : D(i, l) / 2 * 2;
+        const long long ev = l < H ? gxh::dd_fixed(half(gxh::dd_add(at(i, l), at(i, N - l))), lb.sD)
+                                   : gxh::dd_fixed(at(i, l), lb.sD - 1) * 2;
         rest += l < H ? ev : ev / 2;
-        lb.even[i][l] = dig(ev);
+        lb.even[i][l] = digits(ev);
       }
-      if (l < H) lb.odd[i][l] = dig(i < H ? (D(i, l) - D(i, N - l)) / 2 : D(i, l));
+      if (l < H)
+        lb.odd[i][l] = digits(gxh::dd_fixed(i < H ? half(gxh::dd_sub(at(i, l), at(i, N - l))) : at(i, l), lb.sD));
     }
-    if (i < H) lb.even[i][i] = dig(-rest);
+    if (i < H) lb.even[i][i] = digits(-rest);
   }
-  lb.jump = dig((long long)(((__int128)(N * (N + 1)) << lb.sD) / 4));
+  lb.jump = digits(gxh::dd_fixed(gxh::dd_num(N * (N + 1) / 4.), lb.sD));
 }
 
 void lift(dg_ctx* ctx, cudaStream_t st) {
   if constexpr (NP >= 3) {
     gxc::PrecData<double>& P = ctx->d;
-    gx::LiftFxBasis<NP> lb;
-    lift_basis(ctx, lb);
+    const auto& lb = kept<gx::LiftFxBasis<NP>>(ctx->fx_lift, [&](gx::LiftFxBasis<NP>& b) { lift_basis(ctx, b); });
     auto kern = ctx->face_exact ? gx::k_lift_fx<NP, true> : gx::k_lift_fx<NP, false>;
     kern<<<ctx->nElems, gx::LiftFx<NP>::NT, gx::LiftFx<NP>::smem, st>>>(
         P.Pvol.p, P.Met.p, ctx->MetL.p, P.Pf.p, P.Fgeo.p, ctx->E2S.p, lb, P.basis.p, ctx->B.Lhm[0], ctx->nSides, P.Gvol.p,
@@ -105,6 +172,12 @@ void lift(dg_ctx* ctx, cudaStream_t st) {
 }
 
 int configure(const dg_ctx* ctx) {
+  if constexpr (NP >= 4)
+    if (ctx->cfg.split_dg == DG_SPLIT_NONE) {
+      int rc = smem_attr(gx::k_volume_wfx<NP, 0>, gx::VolWfx<NP>::smem, "k_volume_wfx attributes");
+      if (rc == DG_OK) rc = smem_attr(gx::k_volume_wfx<NP, 1>, gx::VolWfx<NP>::smem, "k_volume_wfx attributes");
+      if (rc != DG_OK) return rc;
+    }
   if constexpr (NP >= 3)
     if (ctx->cfg.parabolic && ctx->cfg.node_type == DG_NODETYPE_GAUSS_LOBATTO) {
       int rc = smem_attr(gx::k_lift_fx<NP, true>, gx::LiftFx<NP>::smem, "k_lift_fx attributes");

@@ -86,6 +86,11 @@ int cfg_lift_lines() {
   return DG_OK;
 }
 
+// FP64 weak form: the fixed-point kernel from N = 3 on (48^3 Euler, N = 3: 1.17 against 1.84 ms; 64^3
+// Navier-Stokes, N = 2: 2.97 against 2.65 ms, a block's 27 nodes leave it waiting for its scales)
+template <typename R>
+constexpr bool weak_fx() { return std::is_same<R, double>::value && NP >= 4; }
+
 template <typename R>
 int configure() {
   GX_CUDA_TRY(cudaFuncSetAttribute(gx::k_lift<NP, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lift_smem<R>()),
@@ -97,7 +102,8 @@ int configure() {
               "k_lift carve-out attribute");
   GX_CUDA_TRY(cudaFuncSetAttribute(gx::k_lift<NP, R, 1>, cudaFuncAttributePreferredSharedMemoryCarveout, 100),
               "k_lift carve-out attribute");
-  int rc = cfg_vol<R, -1, 0>() | cfg_vol<R, -1, 1>() | cfg_lift_lines<R>();
+  int rc = cfg_lift_lines<R>();
+  if constexpr (!weak_fx<R>()) rc |= cfg_vol<R, -1, 0>() | cfg_vol<R, -1, 1>();
   if constexpr (NP >= 3) {
     rc |= cfg_vol<R, 0, 0>() | cfg_vol<R, 0, 1>() | cfg_vol<R, 1, 0>() | cfg_vol<R, 1, 1>() | cfg_vol<R, 2, 0>() |
           cfg_vol<R, 2, 1>();
@@ -262,7 +268,10 @@ int rhs(dg_ctx* ctx, PrecData<R>& P, const double* U, gx::RKArgs rk, int rkmode,
   ctx->grad_rho = false;
   int vrc = DG_OK;
   switch (ctx->cfg.split_dg) {
-    case DG_SPLIT_NONE: vrc = vol<R, -1>(ctx, P, U, rk, rkmode, gas, st); break;
+    case DG_SPLIT_NONE:
+      if constexpr (weak_fx<R>()) vrc = GX_CAT(gx_fx_table_, GX_NP).volume(ctx, U, gas, rk, rkmode, st);
+      else vrc = vol<R, -1>(ctx, P, U, rk, rkmode, gas, st);
+      break;
     default:
       if constexpr (NP >= 3) {
         switch (ctx->cfg.split_dg) {

@@ -53,23 +53,23 @@ template <int NP, typename R, int SPLIT, typename S> struct UseVolFx {
 template <int NP> struct VolFxBasis {
   FxLimb Q[NP * NP], iw[NP];
 };
-// MetL[e][3]: log2 of the largest |M_d| (2-norm) of the element, or kFxNoScale where its geometry is outside
+// MetL[e][12]: log2 of the largest |M_d| (2-norm) of the element, then of its largest |M_d,c|, or kFxNoScale where its geometry is outside
 // the range the scales are made for (2^-150 .. 2^150); such elements take the FP64 path
 constexpr float kFxNoScale = 1e9f;
 
-// shifts of one direction (see vol_fx_scales) and the scales of its three kinds of rows: mass, momentum, energy
+// shifts of one direction (see vol_fx_scales) and the scales of its five rows
 struct VolFxShift {
-  int hV, hq, hg, hp, hG, hE;  // left shifts of the products
+  int hV, hq, hg, hp, hG[3], hE;  // left shifts of the products
   int k0, km, kv;              // right shifts: g for the mass row, g for the momentum rows, V for KG's energy row
   int St, kt, Sq, kq;          // viscous fluxes: shift of the product, then right shift (momentum, energy rows)
-  int sM, t[3];                // metric terms * 2^sM; sums * 2^t
+  int sM, t[5];                // metric terms * 2^sM; sums * 2^t
 };
 struct VolFxScale {
   VolFxShift d[3];
-  int s_rho, s_aux, s_p, s_vel, s_tau, s_tq, t[3], ok;
+  int s_rho, s_aux, s_p, s_vel, s_tau, s_tq, t[5], ok;
 };
-// largest magnitudes of the element: fx_mag words; X_U2: float bits of |u|^2
-enum { X_RHO, X_AUX, X_U2, X_P, X_TAU, X_TQ, X_F0, X_FM = X_F0 + 3, X_FE = X_FM + 3, X_NMAX = X_FE + 3,
+// largest magnitudes of the element: fx_mag words; X_U2: float bits of |u|^2; X_F: face fluxes [direction][row]
+enum { X_RHO, X_AUX, X_U2, X_P, X_TAU, X_TQ, X_F, X_V = X_F + 15, X_NMAX,
        X_RHOMIN = X_NMAX, X_PMIN, X_N };
 
 __device__ __forceinline__ float fx_lse(float a, float b) {
@@ -81,7 +81,9 @@ __device__ __forceinline__ float fx_lse(float a, float b) {
 //   mass g;  momentum g us + 4 Q ps Ms + 8 Q fs;  energy g aux_s (+ 2 Q ps V for KG) + 8 Q fs.
 // Products are shifted to use the range up: V, q < 2^61.4, g and the rows' sums of terms < 2^60.4, so that a
 // node's sum over its partners (sum |Q| <= 3.92 for N <= 9, |Q| < 1) and its face flux (< 2^61) stay below
-// 2^63.  Smaller contributions are shifted right to the scale that the largest allows.
+// 2^63.  Smaller contributions are shifted right to the scale that the largest allows.  The momentum rows c of a
+// direction differ in their pressure term p M_d,c (flat elements: a direction's large metric terms meet p in one
+// row only), so each row has its own last shift.
 template <int SPLIT, int PARAB>
 __device__ __forceinline__ void vol_fx_scales(const unsigned* mag, const float* MetL, VolFxScale& S, int lane) {
   const int d = min(lane, 2);
@@ -89,6 +91,7 @@ __device__ __forceinline__ void vol_fx_scales(const unsigned* mag, const float* 
   for (int c = 0; c < X_NMAX; ++c) ok = ok && (c == X_U2 || mag[c] < ((c < X_TAU ? 1022u + 150u : 1022u + 600u) << 20));
   const unsigned lowest = (1022u - 150u) << 20;
   ok = ok && mag[X_RHOMIN] > lowest && mag[X_PMIN] > lowest && mag[X_AUX] > lowest && mag[X_U2] < 0x7b000000u;
+  ok = ok && (mag[X_V] == 0u || mag[X_V] >= (1023u - 60u) << 20);  // the range of fx_float
   ok = ok && (mag[X_RHO] >> 20) - (mag[X_RHOMIN] >> 20) <= 8 && (mag[X_P] >> 20) - (mag[X_PMIN] >> 20) <= 8;
   const float Lr = fx_log2(mag[X_RHO]), La = fx_log2(mag[X_AUX]), Lp = fx_log2(mag[X_P]);
   const float Lu = 0.5f * __log2f(__uint_as_float(mag[X_U2])) + 1e-4f, LM = ok ? MetL[d] : 0.f;
@@ -106,18 +109,29 @@ __device__ __forceinline__ void vol_fx_scales(const unsigned* mag, const float* 
   const int sg = (int)floorf(60.4f - Lqq);
   o.hg = sg - (sq - 2);
   // momentum rows
-  float Lm = fx_lse(Lqq + 1.f + Lu, 4.f + Lp + LM);
-  if (PARAB) Lm = fx_lse(Lm, 4.f + LM + Lt);
-  const int tm = (int)floorf(fminf(60.4f - Lm, 58.f - fx_log2(mag[X_FM + d])));
+  int tm[3], tlow = 100000;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    float Lm = fx_lse(Lqq + 1.f + Lu, 4.f + Lp + (ok ? MetL[3 + 3 * d + c] : 0.f));
+    if (PARAB) Lm = fx_lse(Lm, 4.f + LM + Lt);
+    tm[c] = (int)floorf(fminf(60.4f - Lm, 58.f - fx_log2(mag[X_F + 5 * d + 1 + c])));
+    tlow = min(tlow, tm[c]);
+  }
   const int spx = (int)floorf(59.9f - Lp);
-  o.hG = max(2, max(tm - (sg + s_vel - 64), tm + 2 - (spx + sM - 64)));
-  o.km = min(sg + s_vel - 64 + o.hG - tm, 63);
-  const int sp = tm + 2 - (sM - 64) - o.hG;
+  // the shift of the row with the smallest scale; the others' are larger by their difference
+  const int hl = max(2, max(tlow - (sg + s_vel - 64), tlow + 2 - (spx + sM - 64)));
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    tm[c] = min(tm[c], tlow + 31 - hl);
+    o.hG[c] = hl + tm[c] - tlow;
+  }
+  o.km = min(sg + s_vel - 64 + hl - tlow, 63);
+  const int sp = tlow + 2 - (sM - 64) - hl;
   // energy row
   float Le = Lqq + 1.f + La;
   if (SPLIT == DG_SPLIT_KG) Le = fx_lse(Le, 2.f + Lp + LV);
   if (PARAB) Le = fx_lse(Le, 4.f + LM + Lq);
-  const int t4 = (int)floorf(fminf(60.4f - Le, 58.f - fx_log2(mag[X_FE + d])));
+  const int t4 = (int)floorf(fminf(60.4f - Le, 58.f - fx_log2(mag[X_F + 5 * d + 4])));
   const int he = SPLIT == DG_SPLIT_KG ? max(2, t4 + 65 - sp - sV) : 2;
   // p and aux have one scale for the three directions
   int s_p = min(61 - fx_exp(mag[X_P]), sp + 1), s_aux = min(61 - fx_exp(mag[X_AUX]), t4 - sg + 64 - he);
@@ -130,20 +144,20 @@ __device__ __forceinline__ void vol_fx_scales(const unsigned* mag, const float* 
   o.hE = t4 - sg - s_aux + 64;
   o.kv = SPLIT == DG_SPLIT_KG ? min(sp + sV - 64 + o.hE - t4 - 1, 63) : 0;
   // viscous fluxes: 8 Q f at the rows' scales, from M tau / 2^64 and M tq / 2^64
-  const int ft = tm + 5 - o.hG - (sM + s_tau - 64), fq = t4 + 5 - o.hE - (sM + s_tq - 64);
+  const int ft = tlow + 5 - hl - (sM + s_tau - 64), fq = t4 + 5 - o.hE - (sM + s_tq - 64);
   o.St = max(1, ft); o.kt = min(o.St - ft, 63);
   o.Sq = max(1, fq); o.kq = min(o.Sq - fq, 63);
   // mass row
-  const int t0 = (int)floorf(fminf((float)sg, 59.f - fx_log2(mag[X_F0 + d])));
+  const int t0 = (int)floorf(fminf((float)sg, 59.f - fx_log2(mag[X_F + 5 * d])));
   o.k0 = min(sg - t0, 63);
-  o.t[0] = t0; o.t[1] = tm; o.t[2] = t4;
+  o.t[0] = t0; o.t[1] = tm[0]; o.t[2] = tm[1]; o.t[3] = tm[2]; o.t[4] = t4;
   auto in = [](int h) { return h >= 1 && h <= 31; };
-  ok = ok && in(o.hV) && in(o.hq) && in(o.hg) && in(o.hp) && in(o.hG) && in(o.hE) && o.km >= 0 && o.k0 >= 0 && o.kv >= 0;
+  ok = ok && in(o.hV) && in(o.hq) && in(o.hg) && in(o.hp) && in(o.hG[0]) && in(o.hG[1]) && in(o.hG[2]) && in(o.hE) && o.km >= 0 && o.k0 >= 0 && o.kv >= 0;
   if (PARAB) ok = ok && in(o.St) && in(o.Sq);
   ok = __all_sync(0xffffffffu, ok);
-  int tr[3];
+  int tr[5];
 #pragma unroll
-  for (int r = 0; r < 3; ++r) {
+  for (int r = 0; r < 5; ++r) {
     tr[r] = o.t[r];
 #pragma unroll
     for (int x = 1; x < 4; x <<= 1) tr[r] = min(tr[r], __shfl_xor_sync(0xffffffffu, tr[r], x));
@@ -151,8 +165,45 @@ __device__ __forceinline__ void vol_fx_scales(const unsigned* mag, const float* 
   if (lane < 3) S.d[d] = o;
   if (lane == 0) {
     S.s_rho = s_rho; S.s_aux = s_aux; S.s_p = s_p; S.s_vel = s_vel; S.s_tau = s_tau; S.s_tq = s_tq;
-    S.t[0] = tr[0]; S.t[1] = tr[1]; S.t[2] = tr[2];
+    for (int r = 0; r < 5; ++r) S.t[r] = tr[r];
     S.ok = ok;
+  }
+}
+// largest magnitudes of an element's face fluxes into out[5 * direction + row].  Large blocks: a warp takes whole
+// groups, one reduction each (24^3, N = 7: the kernel 1.86 ms, 1.88 with every warp in all 15 reductions).  Small
+// blocks: all warps together, five loads in flight (64^3, N = 2: 1.94 against 2.46 ms).
+template <int NP, int NT>
+__device__ __forceinline__ void vol_flux_max(const double* Flux, const int* es, unsigned* out) {
+  constexpr int n2 = NP * NP, NW = NT / 32;
+  auto minus = [](int dir) { return dir == 0 ? L_XI_MINUS : (dir == 1 ? L_ETA_MINUS : L_ZETA_MINUS); };
+  auto plus = [](int dir) { return dir == 0 ? L_XI_PLUS : (dir == 1 ? L_ETA_PLUS : L_ZETA_PLUS); };
+  if constexpr (NP >= 6) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 4
+    for (int g = threadIdx.x >> 5; g < 15; g += NW) {
+      const int dir = g / 5, v = g - 5 * dir;
+      const double* const fm = Flux + ((size_t)es[2 * (minus(dir) - 1)] * 5 + v) * n2;
+      const double* const fp = Flux + ((size_t)es[2 * (plus(dir) - 1)] * 5 + v) * n2;
+      unsigned m = 0u;
+#pragma unroll
+      for (int t = 0; t < n2; t += 32)
+        if (t + lane < n2) m = max(m, max(fx_mag(fm[t + lane]), fx_mag(fp[t + lane])));
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) out[g] = m;
+    }
+  } else {
+#pragma unroll 1
+    for (int dir = 0; dir < 3; ++dir) {
+      unsigned f[5] = {0u, 0u, 0u, 0u, 0u};
+      for (int t = threadIdx.x; t < 2 * n2; t += NT) {
+        const int ls = t < n2 ? minus(dir) : plus(dir);
+        const double* fx = Flux + (size_t)es[2 * (ls - 1)] * 5 * n2 + (t < n2 ? t : t - n2);
+#pragma unroll
+        for (int v = 0; v < 5; ++v) f[v] = max(f[v], fx_mag(fx[v * n2]));
+      }
+#pragma unroll
+      for (int v = 0; v < 5; ++v) fx_block_max(f[v], out + 5 * dir + v);
+    }
   }
 }
 
@@ -250,28 +301,8 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
   // (the values wait in the node's own shared-memory slots as FP64 for the scales: slots 0-5 the node data,
   // 6-14 the stresses)
   {
-    unsigned f[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int t = tid; t < 6 * n2; t += NT) {
-      const int ls = t / n2 + 1, pq = t - (ls - 1) * n2;
-      const double* fx = Flux + (size_t)es[2 * (ls - 1)] * 5 * n2 + pq;
-      const unsigned f0 = fx_mag(fx[0]), fe = fx_mag(fx[4 * n2]);
-      const unsigned fm = max(fx_mag(fx[n2]), max(fx_mag(fx[2 * n2]), fx_mag(fx[3 * n2])));
-      const int dir = ls == L_XI_MINUS || ls == L_XI_PLUS ? 0 : (ls == L_ETA_MINUS || ls == L_ETA_PLUS ? 1 : 2);
-#pragma unroll
-      for (int d = 0; d < 3; ++d)
-        if (d == dir) {
-          f[0][d] = max(f[0][d], f0);
-          f[1][d] = max(f[1][d], fm);
-          f[2][d] = max(f[2][d], fe);
-        }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      fx_block_max(f[0][d], &mag[X_F0 + d]);
-      fx_block_max(f[1][d], &mag[X_FM + d]);
-      fx_block_max(f[2][d], &mag[X_FE + d]);
-    }
-    unsigned m[6] = {0, 0, 0, 0, 0, 0}, rmin = 0xffffffffu, pmin = 0xffffffffu;
+    vol_flux_max<NP, NT>(Flux, es, &mag[X_F]);
+    unsigned m[6] = {0, 0, 0, 0, 0, 0}, mv = 0u, rmin = 0xffffffffu, pmin = 0xffffffffu;
 #pragma unroll 1
     for (int node = tid; node < n3; node += NT) {
       const double* P = Pe + node;
@@ -290,6 +321,7 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
       pmin = min(pmin, fx_mag(p));
       const float u = fx_float(fx_mag(vel[0])), v = fx_float(fx_mag(vel[1])), w = fx_float(fx_mag(vel[2]));
       m[X_U2] = max(m[X_U2], __float_as_uint(u * u + v * v + w * w));
+      mv = max(mv, max(fx_mag(vel[0]), max(fx_mag(vel[1]), fx_mag(vel[2]))));
       if constexpr (PARAB) {
         const double* G = Ge + node;
         const double gx[5] = {0., G[n3], G[2 * n3], G[3 * n3], G[4 * n3]};
@@ -311,11 +343,12 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
     }
 #pragma unroll
     for (int c = 0; c < (PARAB ? 6 : 4); ++c) fx_block_max(m[c], &mag[c]);
+    fx_block_max(mv, &mag[X_V]);
     fx_block_min(rmin, &mag[X_RHOMIN]);
     fx_block_min(pmin, &mag[X_PMIN]);
   }
   __syncthreads();
-  if (warp == 0) vol_fx_scales<SPLIT, PARAB>(mag, MetL + (size_t)e * 3, sc, lane);
+  if (warp == 0) vol_fx_scales<SPLIT, PARAB>(mag, MetL + (size_t)e * 12, sc, lane);
   __syncthreads();
   double* const Us = reinterpret_cast<double*>(smem_raw);  // Ut of the element, [node][5], at the end
   if (sc.ok) {
@@ -420,7 +453,7 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
           G[0] = fx_sar(g, sh.k0);
           if constexpr (PARAB) {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) G[1 + c] = fx_dot(gm, us[c], pq, Ms[c], Q, fvs(c), sh.hG);
+            for (int c = 0; c < 3; ++c) G[1 + c] = fx_dot(gm, us[c], pq, Ms[c], Q, fvs(c), sh.hG[c]);
             const FxLimb f4 = fvs(3);
             if constexpr (SPLIT == DG_SPLIT_KG)
               G[4] = fx_dot(gl, as, pq, fx_limb(fx_sar(fx_unbias64(V, sh.hV), sh.kv)), Q, f4, sh.hE);
@@ -428,7 +461,7 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
               G[4] = fx_dot(gl, as, Q, f4, sh.hE);
           } else {
 #pragma unroll
-            for (int c = 0; c < 3; ++c) G[1 + c] = fx_dot(gm, us[c], pq, Ms[c], sh.hG);
+            for (int c = 0; c < 3; ++c) G[1 + c] = fx_dot(gm, us[c], pq, Ms[c], sh.hG[c]);
             if constexpr (SPLIT == DG_SPLIT_KG)
               G[4] = fx_dot(gl, as, pq, fx_limb(fx_sar(fx_unbias64(V, sh.hV), sh.kv)), sh.hE);
             else
@@ -456,7 +489,7 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
             pair(0, B, sb.Q[pos + TPL + n * pos], G);
 #pragma unroll
             for (int c = 0; c < 5; ++c) {
-              const fx64 x = c == 0 ? G[c] : fx_unbias64(G[c], c == 4 ? sh.hE : sh.hG);
+              const fx64 x = c == 0 ? G[c] : fx_unbias64(G[c], c == 4 ? sh.hE : sh.hG[c - 1]);
               acc[tw][0][c] = fx_add(acc[tw][0][c], x);
               acc[tw][1][c] = fx_sub(acc[tw][1][c], x);
             }
@@ -533,10 +566,9 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
       const double* f = Flux + (size_t)side * 5 * n2 + p + n * q;
       const int dir = ls == L_XI_MINUS || ls == L_XI_PLUS ? 0 : (ls == L_ETA_MINUS || ls == L_ETA_PLUS ? 1 : 2);
       fx64* const o = A + (6 + dir * DS) * n3 + vsw<NP>(face_node(n, ls, a, b, is_minus(ls) ? 0 : N));
-      const int r0 = fx_r0(sc.d[dir].t[0] + 2), rm = fx_r0(sc.d[dir].t[1] + 3), r4 = fx_r0(sc.d[dir].t[2] + 3);
 #pragma unroll
       for (int v = 0; v < 5; ++v) {
-        const fx64 x = fx_from(f[v * n2], v == 0 ? r0 : (v == 4 ? r4 : rm));
+        const fx64 x = fx_from(f[v * n2], fx_r0(sc.d[dir].t[v] + (v == 0 ? 2 : 3)));
         o[v * n3] += flip == 0 ? x : -x;
       }
     }
@@ -554,19 +586,18 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
         const int ch = __double2hiint(c), cl = __double2loint(c);
 #pragma unroll
         for (int v = 0; v < 5; ++v) {
-          const int r = v == 0 ? 0 : (v == 4 ? 2 : 1);
           fx64 m = 0;
           FxLimb x[3];
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
             // to the smallest of the three directions' scales, halved for the range of the sum
-            x[d] = fx_limb(fx_sar(a[(6 + d * DS + v) * n3], min(sc.d[d].t[r] - sc.t[r] + 1, 63)));
+            x[d] = fx_limb(fx_sar(a[(6 + d * DS + v) * n3], min(sc.d[d].t[v] - sc.t[v] + 1, 63)));
             m = fx_mid(x[d], w[d], m);
           }
           fx64 t = m >> 32;
 #pragma unroll
           for (int d = 0; d < 3; ++d) t = fx_mad(x[d].h, w[d].h, t);
-          Us[node * 5 + v] = fx_to_double(t, m) * __hiloint2double(ch - ((sc.t[r] + (v == 0 ? 2 : 3) - 5) << 20), cl);
+          Us[node * 5 + v] = fx_to_double(t, m) * __hiloint2double(ch - ((sc.t[v] + (v == 0 ? 2 : 3) - 5) << 20), cl);
         }
       }
     }

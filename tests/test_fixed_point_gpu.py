@@ -39,7 +39,8 @@ def rel(a, b):
     return float(np.linalg.norm(a - b) / np.linalg.norm(b))
 
 
-FORMS = [("pi", dict(SplitDG="pi", Riemann="roe")), ("kg", dict(SplitDG="kg", Riemann="lf"))]
+FORMS = [("pi", dict(SplitDG="pi", Riemann="roe")), ("kg", dict(SplitDG="kg", Riemann="lf")),
+         ("weak", dict(Riemann="roe")), ("gauss", dict(NodeType="gauss", Riemann="lf"))]
 
 
 @pytest.mark.parametrize("parab", [False, True], ids=["euler", "ns"])
@@ -48,8 +49,9 @@ FORMS = [("pi", dict(SplitDG="pi", Riemann="roe")), ("kg", dict(SplitDG="kg", Ri
 def test_units(N, units, form, kw, parab):
     """Lengths in `units`, velocities in sqrt(units), density in 1/units: every scale moves by its own power."""
     L, V, D = units, math.sqrt(units), 1.0 / units
-    m = gx.Mesh(N, 2, 2, 1, 2, (-math.pi * L,) * 3, (math.pi * L,) * 3, deform=0.0)
-    m1 = gx.Mesh(N, 2, 2, 1, 2, (-math.pi,) * 3, (math.pi,) * 3)
+    nt = 1 if "NodeType" in kw else 2
+    m = gx.Mesh(N, nt, 2, 1, 2, (-math.pi * L,) * 3, (math.pi * L,) * 3, deform=0.0)
+    m1 = gx.Mesh(N, nt, 2, 1, 2, (-math.pi,) * 3, (math.pi,) * 3)
     U = state(m1, "units%d%s" % (N, form)) * np.array([D, D * V, D * V, D * V, D * V * V])
     k = dict(kw, parabolic=True, mu0=2e-3 * D * V * L) if parab else kw
     cfg = gx.config(N=N, R=R, **k)
@@ -57,12 +59,13 @@ def test_units(N, units, form, kw, parab):
 
 
 @pytest.mark.parametrize("what", ["mach0.01", "viscous", "flat", "supersonic"])
+@pytest.mark.parametrize("nodes", ["split", "weak", "gauss"])
 @pytest.mark.parametrize("N", [4, 7])
-def test_dominant_terms(N, what):
+def test_dominant_terms(N, nodes, what):
     lo, hi = (-math.pi,) * 3, (math.pi,) * 3
     if what == "flat":
         lo, hi = (-math.pi, -1e-3, -math.pi), (math.pi, 1e-3, math.pi)
-    m = gx.Mesh(N, 2, 2, 2, 1, lo, hi)
+    m = gx.Mesh(N, 1 if nodes == "gauss" else 2, 2, 2, 1, lo, hi)
     mach = {"mach0.01": 0.01, "supersonic": 3.0}.get(what, 0.3)
     noise = 1e-4 if what == "supersonic" else 1e-2
     U = state(m, what, mach=1.0 if what == "supersonic" else mach, noise=noise)
@@ -70,7 +73,8 @@ def test_dominant_terms(N, what):
         U[..., 4] += 2.0 * np.abs(U[..., 1]) ** 2 / U[..., 0]
         U[..., 4] += 6.0 * U[..., 1] + 18.0 * U[..., 0]  # a uniform velocity on top, exactly
         U[..., 1] += 6.0 * U[..., 0]
-    cfg = gx.config(N=N, R=R, SplitDG="pi", Riemann="roe", parabolic=True, mu0=1.0 if what == "viscous" else 2e-3)
+    cfg = gx.config(N=N, R=R, SplitDG="pi" if nodes == "split" else "none", Riemann="roe", parabolic=True,
+                    NodeType="gauss" if nodes == "gauss" else "gauss-lobatto", mu0=1.0 if what == "viscous" else 2e-3)
     assert rel(gpu_rhs(cfg, m, U), Oracle(cfg, m).rhs(U)) <= 1e-12
 
 
@@ -90,7 +94,7 @@ def test_at_rest():
 @pytest.mark.parametrize("N", [3, 6, 7])
 def test_elements_outside_the_scales(N, what, parab, form, kw):
     """One element with a contrast beyond one scale (or magnitudes below 2^-150) among ordinary ones."""
-    m = gx.Mesh(N, 2, 2, 2, 1, (-math.pi,) * 3, (math.pi,) * 3)
+    m = gx.Mesh(N, 1 if "NodeType" in kw else 2, 2, 2, 1, (-math.pi,) * 3, (math.pi,) * 3)
     U = state(m, "outside" + what)
     x = m.Elem_xGP[1, ..., 0:1] * np.array([1.0])
     s = (x - x.min()) / (x.max() - x.min())
