@@ -125,40 +125,6 @@ int upload_fx_basis(dg_ctx* ctx) {
   return DG_OK;
 }
 
-// SurfElem n of every side equals the metric terms of both elements at their face nodes (Gauss-Lobatto nodes;
-// minus faces: with the opposite sign) to the last bits (2^-51 of SurfElem)
-bool face_metrics_exact(int n, int nElems, const std::vector<double>& met, const std::vector<double>& fgeo,
-                        const std::vector<int>& e2s) {
-  const int N = n - 1, n2 = n * n, n3 = n2 * n;
-  for (size_t e = 0; e < (size_t)nElems; ++e)
-    for (int ls = 1; ls <= 6; ++ls) {
-      const int dir = ls == gx::L_XI_MINUS || ls == gx::L_XI_PLUS ? 0 : (ls == gx::L_ETA_MINUS || ls == gx::L_ETA_PLUS ? 1 : 2);
-      const bool minus = ls == gx::L_XI_MINUS || ls == gx::L_ETA_MINUS || ls == gx::L_ZETA_MINUS;
-      const size_t side = e2s[(e * 6 + ls - 1) * 2];
-      const int flip = e2s[(e * 6 + ls - 1) * 2 + 1];
-      const double sg = (minus ? -1. : 1.) * (flip == 0 ? 1. : -1.);
-      for (int b = 0; b < n; ++b)
-        for (int a = 0; a < n; ++a) {
-          // volume face coordinates -> side node (s2v2_inv)
-          int pp = a, qq = b;
-          if (ls == gx::L_XI_MINUS || ls == gx::L_ZETA_MINUS) { pp = b; qq = a; }
-          else if (ls == gx::L_ETA_PLUS) pp = N - a;
-          int p = pp, q = qq;
-          if (flip == 1) { p = qq; q = pp; }
-          else if (flip == 2) p = N - pp;
-          else if (flip == 3) { p = N - qq; q = N - pp; }
-          else if (flip == 4) q = N - qq;
-          const int l = minus ? 0 : N;
-          const int node = dir == 0 ? l + n * (a + n * b) : (dir == 1 ? a + n * (l + n * b) : a + n * (b + n * l));
-          const double* f = &fgeo[side * 10 * n2 + p + n * q];
-          const double se = f[9 * n2];
-          for (int c = 0; c < 3; ++c)
-            if (!(std::fabs(sg * se * f[c * n2] - met[(e * 10 + 3 * dir + c) * n3 + node]) <= se * 4.5e-16)) return false;
-        }
-    }
-  return true;
-}
-
 int run_rhs(dg_ctx* ctx, const double* U, gx::RKArgs rk, int rkmode, cudaStream_t st) {
   const gxc::NPTable* T = table_for(ctx->n);
   if (!T) { set_error("unsupported N"); return DG_ERR_UNSUPPORTED; }
@@ -662,46 +628,20 @@ int dg_set_mesh(dg_ctx* ctx, int nElems, int nSides, int nBCSides, const double*
   CUDA_TRY(cudaMemcpy(ctx->E2S.p, he2s.data(), he2s.size() * sizeof(int), cudaMemcpyHostToDevice), "upload E2S");
   ctx->MetL.release();
   if (ctx->cfg.precision == DG_PRECISION_FP64) {
-    // log2 of each element's largest |M_d| (2-norm) and |M_d,c|, rounded up, for the fixed-point scales
-    std::vector<float> hl((size_t)nElems * 12);
-    for (size_t e = 0; e < (size_t)nElems; ++e) {
-      const double* m = &met[e * 10 * n3];
-      bool fine = true;
-      double big[12] = {0.};
-      for (int d = 0; d < 3; ++d) {
-        for (int t = 0; t < n3; ++t) {
-          double s = 0.;
-          for (int c = 0; c < 3; ++c) {
-            const double a = m[(3 * d + c) * n3 + t] * m[(3 * d + c) * n3 + t];
-            s += a;
-            big[3 + 3 * d + c] = a > big[3 + 3 * d + c] ? a : big[3 + 3 * d + c];
-          }
-          if (!(s < 1e90)) fine = false;
-          big[d] = s > big[d] ? s : big[d];
-        }
-        if (!(big[d] > 1e-90)) fine = false;
-      }
-      for (int t = 0; t < n3; ++t) {
-        const double sj = std::fabs(m[9 * n3 + t]);
-        if (!(sj > 1e-45 && sj < 1e45)) fine = false;
-      }
-      for (int c = 0; c < 12; ++c)
-        hl[e * 12 + c] = !fine ? gx::kFxNoScale : (big[c] > 1e-90 ? (float)(0.5 * std::log2(big[c]) + 1e-5) : -150.f);
-    }
-    // the fixed-point lifting: one scale for the metric terms of an element's three directions
-    bool flat = false;
-    for (size_t e = 0; e < (size_t)nElems; ++e) {
-      const float* l = &hl[e * 12];
-      const float a = std::fmin(l[0], std::fmin(l[1], l[2])), b = std::fmax(l[0], std::fmax(l[1], l[2]));
-      flat = flat || b - a > 8.f;
-    }
     const dg_config& c = ctx->cfg;
     const bool gl = c.node_type == DG_NODETYPE_GAUSS_LOBATTO;
-    ctx->lift_fx = c.parabolic && gl && ctx->N >= 2 && c.lifting == DG_LIFTING_BR1 && !c.do_weak_lifting &&
-                   !c.do_conservative_lifting && !flat;
-    ctx->face_exact = gl && face_metrics_exact(n, nElems, met, fgeo, he2s);
-    if (!ctx->MetL.alloc(hl.size())) { set_error("cudaMalloc mesh"); return DG_ERR_ALLOC; }
-    CUDA_TRY(cudaMemcpy(ctx->MetL.p, hl.data(), hl.size() * sizeof(float), cudaMemcpyHostToDevice), "upload metric scales");
+    gxc::DBuf<int> flags;
+    if (!ctx->MetL.alloc((size_t)nElems * 16) || !flags.alloc(1)) { set_error("cudaMalloc mesh"); return DG_ERR_ALLOC; }
+    int f = 0;
+    cudaError_t err = cudaMemset(flags.p, 0, sizeof(int));
+    if (err == cudaSuccess) err = gxc::mesh_scales(ctx->d.Met.p, ctx->d.Fgeo.p, ctx->E2S.p, nElems, n, gl, ctx->MetL.p, flags.p);
+    if (err == cudaSuccess) err = cudaMemcpy(&f, flags.p, sizeof(int), cudaMemcpyDeviceToHost);
+    flags.release();
+    CUDA_TRY(err, "metric scales");
+    // (from N = 2 on, where the kernels' figures begin; BR2 with an eta that the scales take)
+    ctx->lift_fx = c.parabolic && ctx->N >= 2 && !c.do_weak_lifting && !c.do_conservative_lifting && !(f & 1) &&
+                   (c.lifting != DG_LIFTING_BR2 || std::fabs(c.eta_br2) <= 1e6);
+    ctx->face_exact = gl && !(f & 2);
   }
   // SideToElem on the device, from the validated ElemToSide: master elem/side, slave elem/side, flip
   std::vector<int> hs2e((size_t)nSides * 5, 0);

@@ -121,14 +121,14 @@ struct dg_ctx {
   long long launches = 0;
   int lines_grid = 0;      // blocks of the persistent line volume kernel (SMs x resident blocks), on first use
   int prolong_grid = 0;    // blocks of the persistent prolongation kernel of the mixed form, on first use
-  // FP64 form, block fixed-point kernels: log2 of the largest |M_d| (3) and |M_d,c| (9) of each element
-  // (kFxNoScale: outside the range of the scales), and the basis as limbs (VolFxBasis)
+  // FP64 form, block fixed-point kernels: log2 of the largest |M_d| (3), |M_d,c| (9), SurfElem and
+  // |sJ| of each element (16 words; kFxNoScale: outside the range of the scales), and the basis as limbs (VolFxBasis)
   gxc::DBuf<float> MetL;
-  bool lift_fx = false;    // fixed-point lifting: BR1, strong non-conservative, Gauss-Lobatto, no element flatter than 2^8
+  bool lift_fx = false;    // fixed-point lifting: strong non-conservative form, no element flatter than 2^8
   bool face_exact = false; // SurfElem n = +-M of both elements' face nodes to the last bits (affine elements)
   gxc::DBuf<int> fxb;
   gxh::BasisDD fxB;        // the basis in double-double (FP64 form)
-  std::vector<unsigned char> fx_lift, fx_weak;  // LiftFxBasis, VolWfxBasis, on first use
+  std::vector<unsigned char> fx_lift, fx_weak;  // LiftFxBasis or LiftGfxBasis, VolWfxBasis, on first use
   gxc::DBuf<int> S2E;      // [side][5]: master elem, master local side, slave elem, slave local side, flip (0-based)
   gxc::DBuf<double> wq;    // 1D quadrature weights (n)
   // tangent-linear operator (R = S = Dual<1>), set up on first use
@@ -197,6 +197,11 @@ struct FxTable {
   // lifting kernel where ctx->lift_fx
   void (*lift)(dg_ctx*, cudaStream_t st);
 };
+
+// MetL of a mesh from its packed geometry; flags (device, zeroed): bit 0 an element is flatter than 2^8, bit 1
+// not face_exact (dg_fx_mesh.cu)
+cudaError_t mesh_scales(const double* Met, const double* Fgeo, const int* E2S, int nElems, int n, bool gl, float* MetL,
+                        int* flags);
 
 // face fluxes of the connected sides in the FP64 form (dg_face_fx.cu); false: solver or central part without
 // a kernel there

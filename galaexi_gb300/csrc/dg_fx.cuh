@@ -94,7 +94,7 @@ __device__ __forceinline__ float fx_float(unsigned mag) {
   return __uint_as_float((mag - (896u << 20)) << 3);
 }
 
-// x * 2^s, towards zero, from r0 = fx_r0(s); |x 2^s| < 2^63.  Zeros and subnormal numbers give 0.
+// x * 2^s, towards zero, from r0 = fx_r0(s); |x 2^s| < 2^63, s < 1022.  Zeros and subnormal numbers give 0.
 __device__ __forceinline__ int fx_r0(int s) { return 64 + 1022 - s; }
 __device__ __forceinline__ fx64 fx_from(double x, int r0) {
   const int hi = __double2hiint(x);
@@ -103,7 +103,7 @@ __device__ __forceinline__ fx64 fx_from(double x, int r0) {
   const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
   const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, 11) << 32) | (lo << 11);
   unsigned long long v;
-  asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(eb == 0 ? 64 : r0 - eb));  // amounts above 63 give 0
+  asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(r0 - eb));  // amounts above 63 give 0
   return hi < 0 ? -(fx64)v : (fx64)v;
 }
 
@@ -153,7 +153,25 @@ struct FxDot {
     return K == 0 ? hh + (m >> 30) : (hh << K) + (m >> (30 - K));
   }
 };
-// x * 2^s towards zero in digits, from r0 = fx_r0(s); |x 2^s| < 2^60
+// the same without the low products, which are below one unit of the sum each: where |a| and |b| use the range
+struct FxDotU {
+  fx64 hh, mid;
+  __device__ __forceinline__ FxDotU() : hh(0), mid(0) {}
+  __device__ __forceinline__ void add(FxDig a, FxDig b) {
+    hh = fx_mad(a.h, b.h, hh);
+    mid = fx_mad(a.l, b.h, fx_mad(a.h, b.l, mid));
+  }
+  __device__ __forceinline__ fx64 sum() const { return hh + (mid >> 30); }
+};
+// digits of x * 2^K, K = max(k, 0) up to 30 (k < 0: of x / 2^-k); |x 2^k| < 2^60
+__device__ __forceinline__ FxDig fd_scaled(fx64 x, int k) {
+  if (k < 0) { x = fx_sar(x, -k); k = 0; }
+  const unsigned lo = (unsigned)x, hi = (unsigned)((unsigned long long)x >> 32);
+  return {(int)__funnelshift_r(lo, hi, 30 - k), (int)((lo << k) & 0x3fffffffu)};
+}
+__device__ __forceinline__ fx64 fd_pack(FxDig a) { return (fx64)(((unsigned long long)(unsigned)a.h << 32) | (unsigned)a.l); }
+__device__ __forceinline__ FxDig fd_unpack(fx64 x) { return {(int)(x >> 32), (int)x}; }
+// x * 2^s towards zero in digits, from r0 = fx_r0(s); |x 2^s| < 2^60, s < 1022
 __device__ __forceinline__ FxDig fd_from(double x, int r0) {
   const int hi = __double2hiint(x);
   const unsigned lo = (unsigned)__double2loint(x);
@@ -161,10 +179,13 @@ __device__ __forceinline__ FxDig fd_from(double x, int r0) {
   const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
   const unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, 11) << 32) | (lo << 11);
   unsigned long long v;
-  asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(eb == 0 ? 64 : r0 - eb));
+  asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(r0 - eb));
   const int sg = (hi >> 31) | 1;
   return {(int)(v >> 30) * sg, (int)((unsigned)v & 0x3fffffffu) * sg};
 }
+// the word of |x| that orders magnitudes of integers, and b with |x| < 2^b for every x whose word is at most mag
+__device__ __forceinline__ unsigned fx_mag64(fx64 x) { return (unsigned)abs((int)(x >> 32)); }
+__device__ __forceinline__ int fx_bits(unsigned mag) { return 64 - __clz((int)(mag + 1u)); }
 // x as a double times 2^k
 __device__ __forceinline__ double fx_scaled(fx64 x, int k) {
   const double d = __ll2double_rn(x);

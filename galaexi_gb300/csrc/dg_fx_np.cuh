@@ -8,6 +8,7 @@
 
 #include "dg_ctx.h"
 #include "dg_lift_fx.cuh"
+#include "dg_lift_gfx.cuh"
 #include "dg_volume_fx.cuh"
 #include "dg_volume_wfx.cuh"
 
@@ -160,8 +161,45 @@ void lift_basis(const dg_ctx* ctx, gx::LiftFxBasis<NP>& lb) {
   lb.jump = digits(gxh::dd_fixed(gxh::dd_num(N * (N + 1) / 4.), lb.sD));
 }
 
+// the basis of k_lift_gfx (LiftGfxBasis)
+void gauss_lift_basis(const dg_ctx* ctx, gx::LiftGfxBasis<NP>& gb) {
+  constexpr int N = NP - 1, H = gx::LiftGfxBasis<NP>::H, HE = gx::LiftGfxBasis<NP>::HE;
+  lift_basis(ctx, gb.d);
+  const gxh::BasisDD& B = ctx->fxB;
+  std::vector<gxh::DD> Lh(NP), LL(NP);
+  for (int i = 0; i < NP; ++i) {
+    Lh[i] = gxh::dd_mul(B.Lp[i], gxh::dd_inv(B.w[i]));
+    LL[i] = gxh::dd_mul(gxh::dd_mul(B.Lp[i], Lh[i]), gxh::dd_num(ctx->cfg.eta_br2));
+  }
+  gb.sL = 58 - exponent(Lh);
+  gb.sT = 58 - exponent(B.Lp);
+  gxh::DD sum = gxh::dd_num(0.);
+  for (const gxh::DD& x : LL) sum = gxh::dd_add(sum, x);
+  gb.sLL = 59 - exponent({sum});  // (all of one sign)
+  auto half = [](gxh::DD a) { return gxh::dd_mul(a, gxh::dd_num(0.5)); };
+  for (int i = 0; i < NP; ++i) {
+    gb.Lh[i] = digits(gxh::dd_fixed(Lh[i], gb.sL));
+    gb.LL[i] = digits(gxh::dd_fixed(LL[i], gb.sLL));
+  }
+  for (int l = 0; l < HE; ++l) {
+    gb.te[l] = digits(gxh::dd_fixed(l < H ? half(gxh::dd_add(B.Lp[l], B.Lp[N - l])) : B.Lp[l], gb.sT));
+    if (l < H) gb.to[l] = digits(gxh::dd_fixed(half(gxh::dd_sub(B.Lp[l], B.Lp[N - l])), gb.sT));
+  }
+}
+
+void lift_general(dg_ctx* ctx, cudaStream_t st) {
+  gxc::PrecData<double>& P = ctx->d;
+  const auto& gb = kept<gx::LiftGfxBasis<NP>>(ctx->fx_lift, [&](gx::LiftGfxBasis<NP>& b) { gauss_lift_basis(ctx, b); });
+  const bool gauss = ctx->cfg.node_type == DG_NODETYPE_GAUSS, br2 = ctx->cfg.lifting == DG_LIFTING_BR2;
+  auto kern = !gauss ? gx::k_lift_gfx<NP, false, true> : (br2 ? gx::k_lift_gfx<NP, true, true> : gx::k_lift_gfx<NP, true, false>);
+  kern<<<ctx->nElems, gx::LiftGfx<NP>::NT, gx::LiftGfx<NP>::smem, st>>>(
+      P.Pvol.p, P.Met.p, ctx->MetL.p, P.Pf.p, P.Fgeo.p, ctx->E2S.p, gb, gxc::dev_basis(P, NP), ctx->cfg.eta_br2,
+      ctx->nSides, P.Gvol.p, P.Gf.p);
+}
+
 void lift(dg_ctx* ctx, cudaStream_t st) {
   if constexpr (NP >= 3) {
+    if (ctx->cfg.node_type == DG_NODETYPE_GAUSS || ctx->cfg.lifting == DG_LIFTING_BR2) return lift_general(ctx, st);
     gxc::PrecData<double>& P = ctx->d;
     const auto& lb = kept<gx::LiftFxBasis<NP>>(ctx->fx_lift, [&](gx::LiftFxBasis<NP>& b) { lift_basis(ctx, b); });
     auto kern = ctx->face_exact ? gx::k_lift_fx<NP, true> : gx::k_lift_fx<NP, false>;
@@ -179,9 +217,16 @@ int configure(const dg_ctx* ctx) {
       if (rc != DG_OK) return rc;
     }
   if constexpr (NP >= 3)
-    if (ctx->cfg.parabolic && ctx->cfg.node_type == DG_NODETYPE_GAUSS_LOBATTO) {
-      int rc = smem_attr(gx::k_lift_fx<NP, true>, gx::LiftFx<NP>::smem, "k_lift_fx attributes");
-      if (rc == DG_OK) rc = smem_attr(gx::k_lift_fx<NP, false>, gx::LiftFx<NP>::smem, "k_lift_fx attributes");
+    if (ctx->cfg.parabolic) {
+      const bool gauss = ctx->cfg.node_type == DG_NODETYPE_GAUSS, br2 = ctx->cfg.lifting == DG_LIFTING_BR2;
+      int rc = DG_OK;
+      if (!gauss && br2) rc = smem_attr(gx::k_lift_gfx<NP, false, true>, gx::LiftGfx<NP>::smem, "k_lift_gfx attributes");
+      else if (br2) rc = smem_attr(gx::k_lift_gfx<NP, true, true>, gx::LiftGfx<NP>::smem, "k_lift_gfx attributes");
+      else if (gauss) rc = smem_attr(gx::k_lift_gfx<NP, true, false>, gx::LiftGfx<NP>::smem, "k_lift_gfx attributes");
+      else {
+        rc = smem_attr(gx::k_lift_fx<NP, true>, gx::LiftFx<NP>::smem, "k_lift_fx attributes");
+        if (rc == DG_OK) rc = smem_attr(gx::k_lift_fx<NP, false>, gx::LiftFx<NP>::smem, "k_lift_fx attributes");
+      }
       if (rc != DG_OK) return rc;
     }
   if constexpr (NP >= 3) {

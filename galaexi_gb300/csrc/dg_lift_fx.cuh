@@ -153,7 +153,7 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
     for (int v = 0; v < 4; ++v) fx_block_max(m[v], &mag[v]);
   }
   __syncthreads();
-  bool ok = MetL[(size_t)e * 12] < 200.f;
+  bool ok = MetL[(size_t)e * 16] < 200.f;
 #pragma unroll
   for (int v = 0; v < 4; ++v) ok = ok && mag[v] < ((1022u + 150u) << 20);
   if (ok) {
@@ -232,7 +232,7 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
     __syncthreads();
   }
   // ---- node by node: sJ M digits (< 2^58), the gradients with 2 bits below the digits' unit, and their traces
-  const float Lmax = fmaxf(MetL[(size_t)e * 12], fmaxf(MetL[(size_t)e * 12 + 1], MetL[(size_t)e * 12 + 2]));
+  const float Lmax = fmaxf(MetL[(size_t)e * 16], fmaxf(MetL[(size_t)e * 16 + 1], MetL[(size_t)e * 16 + 2]));
   const int sM = 59 - ((int)floorf(Lmax) + 1), r_M = fx_r0(sM);
 #pragma unroll 1
   for (int it = 0; it < NPT; ++it) {

@@ -238,7 +238,7 @@ k_volume_wfx(const double* __restrict__ U, const double* __restrict__ Pvol, cons
     fx_block_min(pmin, &mag[W_PMIN]);
   }
   __syncthreads();
-  if (tid < 32) vol_wfx_scales<PARAB>(mag, MetL + (size_t)e * 12, sc, tid);
+  if (tid < 32) vol_wfx_scales<PARAB>(mag, MetL + (size_t)e * 16, sc, tid);
   __syncthreads();
   if (sc.ok) {
     // ---- contravariant fluxes

@@ -40,7 +40,9 @@ def rel(a, b):
 
 
 FORMS = [("pi", dict(SplitDG="pi", Riemann="roe")), ("kg", dict(SplitDG="kg", Riemann="lf")),
-         ("weak", dict(Riemann="roe")), ("gauss", dict(NodeType="gauss", Riemann="lf"))]
+         ("weak", dict(Riemann="roe")), ("gauss", dict(NodeType="gauss", Riemann="lf")),
+         ("gauss_br2", dict(NodeType="gauss", Riemann="lf", Lifting="br2")),
+         ("pi_br2", dict(SplitDG="pi", Riemann="roe", Lifting="br2"))]
 
 
 @pytest.mark.parametrize("parab", [False, True], ids=["euler", "ns"])
