@@ -512,6 +512,9 @@ int dg_ctx_create(const dg_config* cfg, dg_ctx** out) {
   const gxc::NPTable* T = table_for(ctx->n);
   int rc = upload_basis(ctx, ctx->d);
   if (rc == DG_OK && cfg->precision == DG_PRECISION_MIXED) rc = upload_basis(ctx, ctx->f);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    ctx->sms = 0;
   if (rc == DG_OK) rc = (cfg->precision == DG_PRECISION_FP64) ? T->configure_d() : T->configure_f();
   if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64) rc = upload_fx_basis(ctx);
   if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64) rc = fx_table_for(ctx->n)->configure(ctx);

@@ -119,6 +119,7 @@ struct dg_ctx {
   gxc::DBuf<unsigned long long> bad;
   gxc::DBuf<int> kerr;     // set by a kernel whose bounded wait ran out (read by the synchronising calls)
   long long launches = 0;
+  int sms = 0;             // SMs of the device
   int lines_grid = 0;      // blocks of the persistent line volume kernel (SMs x resident blocks), on first use
   int prolong_grid = 0;    // blocks of the persistent prolongation kernel of the mixed form, on first use
   // FP64 form, block fixed-point kernels: log2 of the largest |M_d| (3), |M_d,c| (9), SurfElem and

@@ -121,7 +121,7 @@ int volume_spl(dg_ctx* ctx, const double* U, const gx::Gas<double>& gas, gx::RKA
 
 int volume(dg_ctx* ctx, const double* U, const gx::Gas<double>& gas, gx::RKArgs rk, int rkmode, cudaStream_t st) {
   if (ctx->cfg.split_dg == DG_SPLIT_NONE) {
-    if constexpr (NP >= 4) return volume_weak(ctx, U, gas, rk, rkmode, st);
+    if constexpr (NP >= 3) return volume_weak(ctx, U, gas, rk, rkmode, st);
   }
   if constexpr (NP >= 3)
     return ctx->cfg.split_dg == DG_SPLIT_KG ? volume_spl<DG_SPLIT_KG>(ctx, U, gas, rk, rkmode, st)
@@ -210,7 +210,7 @@ void lift(dg_ctx* ctx, cudaStream_t st) {
 }
 
 int configure(const dg_ctx* ctx) {
-  if constexpr (NP >= 4)
+  if constexpr (NP >= 3)
     if (ctx->cfg.split_dg == DG_SPLIT_NONE) {
       int rc = smem_attr(gx::k_volume_wfx<NP, 0>, gx::VolWfx<NP>::smem, "k_volume_wfx attributes");
       if (rc == DG_OK) rc = smem_attr(gx::k_volume_wfx<NP, 1>, gx::VolWfx<NP>::smem, "k_volume_wfx attributes");

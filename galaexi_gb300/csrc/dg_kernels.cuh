@@ -140,12 +140,18 @@ template <int NP, typename R> struct ProlongMinBlocks {
   static constexpr int v =
       (OffsetOf<R>::v && NP == 6) ? 5 : ((OffsetOf<R>::v && 3 * EPBof<NP>::v * NP * NP * NP <= 2048) ? 3 : 2);
 };
-template <int NP, typename R, typename S = double>
-__global__ void __launch_bounds__(EPBof<NP>::v * NP * NP * NP, ProlongMinBlocks<NP, R>::v)
+// threads of a block of EPB elements: one per node; a single small element (of a mesh that leaves SMs without a
+// block at EPBof elements per block) one per face node too
+template <int NP, int EPB> struct ProlongThreads {
+  static constexpr int n3 = NP * NP * NP, f = 6 * NP * NP;
+  static constexpr int v = EPB == EPBof<NP>::v ? EPB * n3 : ((n3 > f ? n3 : f) + 31) / 32 * 32;
+};
+template <int NP, typename R, typename S = double, int EPB = EPBof<NP>::v>
+__global__ void __launch_bounds__(ProlongThreads<NP, EPB>::v, EPB == EPBof<NP>::v ? ProlongMinBlocks<NP, R>::v : 1)
 k_prolong(const S* __restrict__ U, const int* __restrict__ E2S, const double* __restrict__ Lm,
           const double* __restrict__ Lp, Gas<R> gas, Launch L, R* __restrict__ Pvol, R* __restrict__ Uf,
           R* __restrict__ Pf) {
-  constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP, EPB = EPBof<NP>::v, N = NP - 1;
+  constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP, N = NP - 1;
   // mixed form: FP32 copies of density and momenta (converted once per node; Gauss nodes interpolate
   // them to the faces in FP32), the energy in FP64.  Static shared memory is limited to 48 KB, so N = 9
   // keeps the plain FP64 interpolation.

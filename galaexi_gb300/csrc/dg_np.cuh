@@ -86,10 +86,13 @@ int cfg_lift_lines() {
   return DG_OK;
 }
 
-// FP64 weak form: the fixed-point kernel from N = 3 on (48^3 Euler, N = 3: 1.17 against 1.84 ms; 64^3
-// Navier-Stokes, N = 2: 2.97 against 2.65 ms, a block's 27 nodes leave it waiting for its scales)
+// FP64 weak form: the fixed-point kernel from N = 3 on (48^3 Euler, N = 3: 1.16 against 1.84 ms).  At N = 2 a block's
+// 27 nodes leave it waiting for its scales: it is the faster one (Navier-Stokes, 4^3 elements 16 against 22 us, 12^3
+// 33 against 37) only as long as the SMs hold all elements at once, kWeakFxResident blocks each; then 16^3 elements
+// take 59 against 53 us, 64^3 2.97 against 2.65 ms
+constexpr int kWeakFxResident = 10;
 template <typename R>
-constexpr bool weak_fx() { return std::is_same<R, double>::value && NP >= 4; }
+constexpr bool weak_fx() { return std::is_same<R, double>::value && NP >= 3; }
 
 template <typename R>
 int configure() {
@@ -103,7 +106,7 @@ int configure() {
   GX_CUDA_TRY(cudaFuncSetAttribute(gx::k_lift<NP, R, 1>, cudaFuncAttributePreferredSharedMemoryCarveout, 100),
               "k_lift carve-out attribute");
   int rc = cfg_lift_lines<R>();
-  if constexpr (!weak_fx<R>()) rc |= cfg_vol<R, -1, 0>() | cfg_vol<R, -1, 1>();
+  if constexpr (!weak_fx<R>() || NP == 3) rc |= cfg_vol<R, -1, 0>() | cfg_vol<R, -1, 1>();
   if constexpr (NP >= 3) {
     rc |= cfg_vol<R, 0, 0>() | cfg_vol<R, 0, 1>() | cfg_vol<R, 1, 0>() | cfg_vol<R, 1, 1>() | cfg_vol<R, 2, 0>() |
           cfg_vol<R, 2, 1>();
@@ -194,6 +197,15 @@ void rhs_front(dg_ctx* ctx, PrecData<R>& P, const S* U, const gx::Gas<R>& gas, c
       persistent = true;
     }
   }
+  if constexpr (EPB > 1 && std::is_same<S, double>::value) {
+    // fewer blocks than SMs: one element per block (4^3 elements, N = 2: 11.5 against 16.4 us; 8^3, N = 3: 12.7 against
+    // 14.9; at 10^3, N = 3, the two are equal)
+    if (!persistent && grid < ctx->sms) {
+      gx::k_prolong<NP, R, S, 1><<<ctx->nElems, gx::ProlongThreads<NP, 1>::v, 0, st>>>(U, ctx->E2S.p, bd.Lm, bd.Lp, gas, L,
+                                                                                      P.Pvol.p, P.Uf.p, P.Pf.p);
+      persistent = true;
+    }
+  }
   if (!persistent)
     gx::k_prolong<NP, R, S><<<grid, NT, 0, st>>>(U, ctx->E2S.p, bd.Lm, bd.Lp, gas, L, P.Pvol.p, P.Uf.p, P.Pf.p);
   ctx->launches++;
@@ -269,8 +281,13 @@ int rhs(dg_ctx* ctx, PrecData<R>& P, const double* U, gx::RKArgs rk, int rkmode,
   int vrc = DG_OK;
   switch (ctx->cfg.split_dg) {
     case DG_SPLIT_NONE:
-      if constexpr (weak_fx<R>()) vrc = GX_CAT(gx_fx_table_, GX_NP).volume(ctx, U, gas, rk, rkmode, st);
-      else vrc = vol<R, -1>(ctx, P, U, rk, rkmode, gas, st);
+      if constexpr (weak_fx<R>()) {
+        if (NP >= 4 || ctx->nElems <= kWeakFxResident * ctx->sms) {
+          vrc = GX_CAT(gx_fx_table_, GX_NP).volume(ctx, U, gas, rk, rkmode, st);
+          break;
+        }
+      }
+      vrc = vol<R, -1>(ctx, P, U, rk, rkmode, gas, st);
       break;
     default:
       if constexpr (NP >= 3) {
