@@ -1146,7 +1146,23 @@ __device__ __forceinline__ void atomic_min_pos(double* addr, double val) {
   atomicMin(a, v);
 }
 
-// one block per element, blockDim = n^3 rounded up to a warp multiple
+// Doubles as integers of the same order, NaN below all, and back: the maxima of k_cfl (fmax's: a number before a
+// NaN) are taken on the integer pipes, where a 64-bit FP64 maximum costs a comparison of 65 cycles
+__device__ __forceinline__ long long order_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return (b & 0x7fffffffffffffffll) > 0x7ff0000000000000ll ? (long long)(1ull << 63) : (b < 0 ? b ^ 0x7fffffffffffffffll : b);
+}
+__device__ __forceinline__ double order_value(long long k) { return __longlong_as_double(k < 0 ? k ^ 0x7fffffffffffffffll : k); }
+// the largest key of a warp: the upper words, then the lower ones of those that have the largest
+__device__ __forceinline__ long long warp_max_key(long long k) {
+  const int h = (int)(k >> 32), m = __reduce_max_sync(0xffffffffu, h);
+  const unsigned l = __reduce_max_sync(0xffffffffu, h == m ? (unsigned)k : 0u);
+  return ((long long)m << 32) | l;
+}
+
+// one block per element, blockDim = n^3 rounded up to a warp multiple; bound by FP64 issue (about 50 instructions per
+// node; the six maxima by fmax took as long again: the whole call with 24^3 elements at N = 7 1203 us, now 737, with
+// 8^3 elements 104 and 83)
 template <int NP>
 __global__ void __launch_bounds__(1024)
 k_cfl(const double* __restrict__ U, const double* __restrict__ MetD, const double* __restrict__ Cm, int nElems,
@@ -1154,7 +1170,7 @@ k_cfl(const double* __restrict__ U, const double* __restrict__ MetD, const doubl
       unsigned long long* __restrict__ bad) {
   constexpr int n3 = NP * NP * NP;
   constexpr int NW = (n3 + 31) / 32;
-  __shared__ double red[6][NW];
+  __shared__ long long red[6][NW];
   const int e = blockIdx.x;
   const int node = threadIdx.x;
   double lam[6] = {0, 0, 0, 0, 0, 0};
@@ -1176,22 +1192,23 @@ k_cfl(const double* __restrict__ U, const double* __restrict__ MetD, const doubl
       if (parabolic) lam[3 + d] = mu0 * srho * C[(3 + d) * n3];
     }
   }
-  // max over the element's nodes: warp shuffle, then across the element's warps
+  // max over the element's nodes: of each warp, then of the element's warps
 #pragma unroll
   for (int d = 0; d < 6; ++d) {
-    double v = lam[d];
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) red[d][threadIdx.x >> 5] = v;
+    const long long k = warp_max_key(order_key(lam[d]));
+    if ((threadIdx.x & 31) == 0) red[d][threadIdx.x >> 5] = k;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     double mx[6];
-    for (int d = 0; d < 6; ++d) {
-      mx[d] = red[d][0];
-      for (int w = 1; w < NW; ++w) mx[d] = fmax(mx[d], red[d][w]);
-    }
-    atomic_min_pos(dt2, CFLScale * 2. / (mx[0] + mx[1] + mx[2]));
-    if (parabolic) atomic_min_pos(dt2 + 1, DFLScale * 4. / (mx[3] + mx[4] + mx[5]));
+#pragma unroll
+    for (int d = 0; d < 6; ++d)
+      mx[d] = order_value(warp_max_key((int)threadIdx.x < NW ? red[d][threadIdx.x] : (long long)(1ull << 63)));
+    // lane 0: advection, lane 1: viscosity
+    const int g = threadIdx.x;
+    if (g == 0 || (g == 1 && parabolic))
+      atomic_min_pos(dt2 + g, (g == 0 ? CFLScale * 2. : DFLScale * 4.) /
+                                  (g == 0 ? mx[0] + mx[1] + mx[2] : mx[3] + mx[4] + mx[5]));
   }
 }
 
