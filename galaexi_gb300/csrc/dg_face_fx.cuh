@@ -17,65 +17,10 @@
 //   * Roe's wave strengths from the jumps of the conserved variables, in vector form;
 //   * the viscous traction tau n from the symmetrised gradient, its momentum part added up over both sides.
 #pragma once
+#include "dg_dp.cuh"
 #include "dg_kernels.cuh"
 
 namespace gx {
-
-__device__ __forceinline__ long long dp_bits(double x) { return __double_as_longlong(x); }
-__device__ __forceinline__ double dp_abs(double x) { return __hiloint2double(__double2hiint(x) & 0x7fffffff, __double2loint(x)); }
-// the larger of two numbers of which at most one is negative; as fmax, a number before a NaN
-__device__ __forceinline__ double dp_max(double a, double b) {
-  const long long x = dp_bits(a), y = dp_bits(b), inf = 0x7ff0000000000000ll;
-  return (x > y && x <= inf) || y > inf ? a : b;
-}
-// x >= 0 and x <= 0 (signed zeros aside), false for NaN
-__device__ __forceinline__ bool dp_ge0(double x) { return (unsigned)__double2hiint(x) <= 0x7ff00000u; }
-__device__ __forceinline__ bool dp_le0(double x) {
-  const unsigned h = (unsigned)__double2hiint(x);
-  return h >= 0x80000000u && h <= 0xfff00000u;
-}
-// x * 2^k where neither leaves the normal range
-__device__ __forceinline__ double dp_scale(double x, int k) { return __hiloint2double(__double2hiint(x) + (k << 20), __double2loint(x)); }
-// a positive float in [2^-126, 2^127] times 2^k as a double, by integer instructions
-__device__ __forceinline__ double dp_widen(float f, int k) {
-  const int b = __float_as_int(f);
-  return __hiloint2double((((b >> 23) + 1023 - 127 + k) << 20) | ((b & 0x7fffff) >> 3), b << 29);
-}
-__device__ __noinline__ double dp_rcp_rare(double x) { return 1. / x; }
-__device__ __noinline__ double dp_div_rare(double a, double b) { return a / b; }
-__device__ __noinline__ double dp_rsqrt_rare(double x) { return 1. / sqrt(x); }
-
-// 1/x: Newton-Raphson r <- r + r (1 - x r) from the 22-bit FP32 approximation of the mantissa's reciprocal
-__device__ __forceinline__ double dp_rcp(double x) {
-  const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
-  if ((unsigned)(e - 123) >= 1800u) return dp_rcp_rare(x);  // zero, subnormal, huge, infinite, NaN
-  const float m = __int_as_float(0x3f800000 | ((hi & 0xfffff) << 3) | (int)((unsigned)__double2loint(x) >> 29));
-  double r = dp_widen(__fdividef(1.f, m), 1023 - e);
-  r = __hiloint2double(__double2hiint(r) | (hi & 0x80000000), __double2loint(r));
-  r = fma(r, fma(-x, r, 1.), r);
-  return fma(r, fma(-x, r, 1.), r);
-}
-// a/b with the remainder of the first quotient
-__device__ __forceinline__ double dp_div(double a, double b) {
-  if ((unsigned)(((__double2hiint(b) >> 20) & 0x7ff) - 123) >= 1800u) return dp_div_rare(a, b);
-  const double r = dp_rcp(b), q = a * r;
-  return fma(fma(-b, q, a), r, q);
-}
-// 1/sqrt(x) for x > 0: Newton's iteration y <- y + y/2 (1 - x y y) from the FP32 approximation
-__device__ __forceinline__ double dp_rsqrt(double x) {
-  const int hi = __double2hiint(x);
-  if ((unsigned)((hi >> 20) - 123) >= 1800u) return dp_rsqrt_rare(x);  // also every negative x
-  const int e = (hi >> 20) - 1023, k = e >> 1;  // x = m 2^(2k), 1 <= m < 4
-  const float m = __int_as_float(((127 + (e - 2 * k)) << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)__double2loint(x) >> 29));
-  double y = dp_widen(rsqrtf(m), -k);
-  y = fma(dp_scale(y, -1), fma(-(x * y), y, 1.), y);
-  return fma(dp_scale(y, -1), fma(-(x * y), y, 1.), y);
-}
-// sqrt(x) from y = 1/sqrt(x), with the remainder of x y
-__device__ __forceinline__ double dp_sqrt_from(double x, double y) {
-  const double s = x * y;
-  return fma(fma(-s, s, x), dp_scale(y, -1), s);
-}
 
 struct FaceGas {
   double kappaM1, kR, mu, lambda;  // kR = kappa R

@@ -7,6 +7,7 @@
 // followed by a metric contraction.  All are branch-uniform within a launch (the solver and
 // split choice are launch constants).
 #pragma once
+#include "dg_dp.cuh"
 #include <cuda_runtime.h>
 #include <math.h>
 #include <type_traits>
@@ -64,7 +65,8 @@ __device__ __forceinline__ void cons_to_prim_mixed(const R c[4], double E, const
 template <typename R, typename S>
 __device__ __forceinline__ void cons_to_prim_d(const S u[5], const Gas<R>& g, R prim[6], R& srho) {
   if constexpr (!OffsetOf<R>::v) {
-    srho = R(1) / (R)u[0];
+    if constexpr (std::is_same<R, double>::value) srho = dp_rcp((R)u[0]);  // four FP64 instructions fewer than the division
+    else srho = R(1) / (R)u[0];
     prim[0] = (R)u[0];
     prim[1] = (R)u[1] * srho;
     prim[2] = (R)u[2] * srho;

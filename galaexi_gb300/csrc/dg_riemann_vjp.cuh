@@ -14,7 +14,7 @@ namespace gx {
 __device__ __forceinline__ void prim_vjp(const double U[5], double kappaM1, double sR, double rb, double ub,
                                          double vb, double wb, double pb, double Tb, double srhob, double Eb,
                                          double m1b, double m2b, double m3b, double Ub[5]) {
-  const double srho = 1. / U[0];
+  const double srho = dp_rcp(U[0]);
   const double vel[3] = {U[1] * srho, U[2] * srho, U[3] * srho};
   const double p = kappaM1 * (U[4] - 0.5 * (U[1] * vel[0] + U[2] * vel[1] + U[3] * vel[2]));
   // T = p * srho / R
