@@ -129,6 +129,9 @@ template <int NP> struct EPBof { static constexpr int v = (NP * NP * NP >= 128) 
 // later the surface flux vectors of one normal direction (2 faces x 15 x n^2)
 __host__ __device__ constexpr int lift_ps_slots(int NP) { return 5 * NP * NP * NP > 30 * NP * NP ? 5 * NP * NP * NP : 30 * NP * NP; }
 
+// the FP32 form of k_lift holds the surface flux vectors of all six faces beside the others (Gauss nodes and BR2)
+template <int NP, typename R> __host__ __device__ constexpr bool lift_all_faces() { return sizeof(R) == 4 && NP >= 3 && NP <= 9; }
+
 // =====================================================================================
 // k_prolong: ConsToPrim_Volume + ProlongToFace_CUDA + GetPrimitiveStateSurface.  At least two
 // blocks per SM for the FP64 form (FP64-issue bound); three for the mixed form up to N = 7, whose FP64
@@ -330,6 +333,8 @@ template <int NP, typename R> struct LiftMinBlocks {
       (sizeof(R) == 4 && EPBof<NP>::v * NP * NP * NP <= 256) ? (EPBof<NP>::v == 1 ? 5 : 4) : 2;
 };
 
+template <typename R> __device__ __forceinline__ R* smem_raw_as(unsigned char* p) { return reinterpret_cast<R*>(p); }
+
 template <int NP, typename R, int V0 = 0>
 __global__ void __launch_bounds__(EPBof<NP>::v * NP * NP * NP, LiftMinBlocks<NP, R>::v)
 k_lift(const R* __restrict__ Pvol, const R* __restrict__ Met, const R* __restrict__ Pf, const R* __restrict__ Fgeo,
@@ -351,7 +356,7 @@ k_lift(const R* __restrict__ Pvol, const R* __restrict__ Met, const R* __restric
       const R* m = Met + (size_t)e0 * 10 * n3;
       if (bulk_ok(m, m, 10 * n3 * sizeof(R))) bulk_prefetch_l2(m, 10 * n3 * sizeof(R));
     }
-    if (threadIdx.x >= 64 && threadIdx.x < 70 && nloc > 0) {
+    if (facepass && threadIdx.x >= 64 && threadIdx.x < 70 && nloc > 0) {
       const size_t side = (size_t)E2S[((size_t)e0 * 6 + threadIdx.x - 64) * 2];
       const R* pm = Pf + side * 6 * n2;
       const R* ps = Pf + ((size_t)L.nSides + side) * 6 * n2;
@@ -364,6 +369,45 @@ k_lift(const R* __restrict__ Pvol, const R* __restrict__ Met, const R* __restric
     }
   }
   const R sigflux = (L.lift_mode == 2) ? R(1) : R(-1);
+  constexpr bool ALLF = lift_all_faces<NP, R>();
+  constexpr int NF = ALLF ? 3 * (5 - V0) : 15;  // components held
+  auto comp = [](int d, int v) { return ALLF ? d * (5 - V0) + v - V0 : d * 5 + v; };
+  // surface flux vector F = 0.5*SurfElem*flux*n of a face node, component comp(d, v) to out[comp * n2]
+  auto face_flux = [&](int ef, int ls, int ab, R* out) {
+    const int side = E2S[(ef * 6 + ls - 1) * 2 + 0];
+    const int flip = E2S[(ef * 6 + ls - 1) * 2 + 1];
+    int p, q;
+    s2v2_inv(N, ab % n, ab / n, flip, ls, p, q);
+    const int pq = p + n * q;
+    const R* pm = Pf + (size_t)side * 6 * n2 + pq;
+    const R* ps = Pf + ((size_t)L.nSides + side) * 6 * n2 + pq;
+    const R* fg = Fgeo + (size_t)side * 10 * n2 + pq;
+    const R sig = (L.lift_mode == 2) ? ((flip == 0) ? R(1) : R(-1)) : R(1);
+    const R wgt = sig * R(0.5) * fg[9 * n2];
+    const R nvv[3] = {wgt * fg[0], wgt * fg[n2], wgt * fg[2 * n2]};
+#pragma unroll
+    for (int v = V0; v < 5; ++v) {
+      const int c = liftc[v];
+      const R fl = sigflux * pm[c * n2] + ps[c * n2];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) out[comp(d, v) * n2] = fl * nvv[d];
+    }
+  };
+  auto face_side = [](int dir, int mp) {
+    return dir == 0 ? (mp == 0 ? L_XI_MINUS : L_XI_PLUS)
+                    : (dir == 1 ? (mp == 0 ? L_ETA_MINUS : L_ETA_PLUS) : (mp == 0 ? L_ZETA_MINUS : L_ZETA_PLUS));
+  };
+  R* const Fa = smem_raw_as<R>(smem_raw) + (size_t)EPB * (lift_ps_slots(NP) + 15 * n3);  // [EPB][6][NF][n2] (ALLF)
+  if constexpr (ALLF) {
+    // FP32 form: the face nodes of all six faces at once, while the primitives are on their way; one normal direction
+    // per pass left two thirds of the threads idle at six barriers (20^3 curved elements, N = 5, BR2: 250 against
+    // 232 us).  At N = 9 the six faces' vectors leave one block per SM: 514 against 325 us.
+    if (!facepass)
+      for (int t = threadIdx.x; t < nloc * 6 * n2; t += blockDim.x) {
+        const int fe = t / (6 * n2), r = t - fe * 6 * n2, f = r / n2, ab = r - f * n2;
+        face_flux(e0 + fe, face_side(f >> 1, f & 1), ab, Fa + ((size_t)fe * 6 + f) * NF * n2 + ab);
+      }
+  }
   for (int t = threadIdx.x; t < nloc * 5 * n3; t += blockDim.x) {
     int el = t / (5 * n3), r = t - el * 5 * n3;
     int c = r / n3, node = r - c * n3;
@@ -487,55 +531,36 @@ k_lift(const R* __restrict__ Pvol, const R* __restrict__ Met, const R* __restric
     // their node into shared memory (over the lifted primitives, which are no longer read), then every
     // node adds sJ*(Lhat_minus(l)*F_minus + Lhat_plus(l)*F_plus) of its line (Gauss nodes) or of its
     // face (Gauss-Lobatto nodes, BR2).  Each face node's data is read from global memory once.
-    R (*Fs)[2][15][n2] = reinterpret_cast<R (*)[2][15][n2]>(smem_raw);  // [EPB][minus/plus][15][n2]
+    R* const Fd = ALLF ? Fa : smem_raw_as<R>(smem_raw);
+    constexpr int FE = ALLF ? 6 : 2;  // faces held
 #pragma unroll 1
     for (int dir = 0; dir < 3; ++dir) {
-      __syncthreads();
-      for (int t = threadIdx.x; t < nloc * 2 * n2; t += blockDim.x) {
-        const int fe = t / (2 * n2), r = t - fe * 2 * n2;
-        const int mp = r < n2 ? 0 : 1;
-        const int ab = r - mp * n2;
-        const int a = ab % n, b = ab / n;
-        const int ls = dir == 0 ? (mp == 0 ? L_XI_MINUS : L_XI_PLUS)
-                                : (dir == 1 ? (mp == 0 ? L_ETA_MINUS : L_ETA_PLUS) : (mp == 0 ? L_ZETA_MINUS : L_ZETA_PLUS));
-        const int ef = e0 + fe;
-        const int side = E2S[(ef * 6 + ls - 1) * 2 + 0];
-        const int flip = E2S[(ef * 6 + ls - 1) * 2 + 1];
-        int p, q;
-        s2v2_inv(N, a, b, flip, ls, p, q);
-        const int pq = p + n * q;
-        const R* pm = Pf + (size_t)side * 6 * n2 + pq;
-        const R* ps = Pf + ((size_t)L.nSides + side) * 6 * n2 + pq;
-        const R* fg = Fgeo + (size_t)side * 10 * n2 + pq;
-        const R sig = (L.lift_mode == 2) ? ((flip == 0) ? R(1) : R(-1)) : R(1);
-        const R wgt = sig * R(0.5) * fg[9 * n2];
-        const R nvv[3] = {wgt * fg[0], wgt * fg[n2], wgt * fg[2 * n2]};
-#pragma unroll
-        for (int v = V0; v < 5; ++v) {
-          const int c = liftc[v];
-          const R fl = sigflux * pm[c * n2] + ps[c * n2];
-#pragma unroll
-          for (int d = 0; d < 3; ++d) Fs[fe][mp][d * 5 + v][ab] = fl * nvv[d];
+      if constexpr (!ALLF) {
+        __syncthreads();
+        for (int t = threadIdx.x; t < nloc * 2 * n2; t += blockDim.x) {
+          const int fe = t / (2 * n2), r = t - fe * 2 * n2, mp = r < n2 ? 0 : 1, ab = r - mp * n2;
+          face_flux(e0 + fe, face_side(dir, mp), ab, Fd + ((size_t)fe * 2 + mp) * NF * n2 + ab);
         }
+        __syncthreads();
       }
-      __syncthreads();
       if (act) {
         const int a = dir == 0 ? j : i, b = dir == 2 ? j : k, l = dir == 0 ? i : (dir == 1 ? j : k);
-        const int ab = a + n * b;
+        const R* const Fm = Fd + ((size_t)el * FE + (ALLF ? 2 * dir : 0)) * NF * n2 + a + n * b;
+        const R* const Fp = Fm + NF * n2;
         if (L.gauss) {
           const R cm = sj * sb.Lhm[l], cp = sj * sb.Lhp[l];
 #pragma unroll
           for (int d = 0; d < 3; ++d)
 #pragma unroll
             for (int v = V0; v < 5; ++v)
-              g[d][v] = g[d][v] + cm * Fs[el][0][d * 5 + v][ab] + cp * Fs[el][1][d * 5 + v][ab];
+              g[d][v] = g[d][v] + cm * Fm[comp(d, v) * n2] + cp * Fp[comp(d, v) * n2];
         } else if (l == 0 || l == N) {
-          const int mp = l == 0 ? 0 : 1;
+          const R* const Fl = l == 0 ? Fm : Fp;
           const R cf = sj * (l == 0 ? sb.Lhm[0] : sb.Lhp[N]);
 #pragma unroll
           for (int d = 0; d < 3; ++d)
 #pragma unroll
-            for (int v = V0; v < 5; ++v) g[d][v] = g[d][v] + cf * Fs[el][mp][d * 5 + v][ab];
+            for (int v = V0; v < 5; ++v) g[d][v] = g[d][v] + cf * Fl[comp(d, v) * n2];
         }
       }
     }
@@ -582,22 +607,28 @@ k_lift(const R* __restrict__ Pvol, const R* __restrict__ Met, const R* __restric
       pm = Pf + (size_t)side * 6 * n2 + pq;
       ps = Pf + ((size_t)L.nSides + side) * 6 * n2 + pq;
     }
-    for (int c = 0; c < 15; ++c) {
-      if (c % 5 < V0) continue;
-      R s;
-      if (!L.gauss) {
-        s = Gs[el][c][vsw<NP>(face_node(n, ls, a, b, is_minus(ls) ? 0 : N))];
-      } else {
-        const R* Lv = is_minus(ls) ? sb.Lm : sb.Lp;
-        s = Gs[el][c][vsw<NP>(face_node(n, ls, a, b, 0))] * Lv[0];
+    // (line offsets, jumps and geometry once for the twelve components, whose loop is unrolled: 20^3 curved elements,
+    // N = 5, FP32 form, BR2 232 -> 140 us for the kernel, N = 7, 16^3 291 -> 158)
+    const int x0 = face_node(n, ls, a, b, 0), xs = face_node(n, ls, a, b, 1) - x0;
+    const int xe = face_node(n, ls, a, b, is_minus(ls) ? 0 : N);
+    const R* Lv = is_minus(ls) ? sb.Lm : sb.Lp;
 #pragma unroll
-        for (int l = 1; l < n; ++l) s = s + Gs[el][c][vsw<NP>(face_node(n, ls, a, b, l))] * Lv[l];
+    for (int v = V0; v < 5; ++v) {
+      const R jump = L.br2 ? bw * (ps[liftc[v] * n2] - pm[liftc[v] * n2]) : R(0);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const R* const G = Gs[el][d * 5 + v];
+        R s;
+        if (!L.gauss) {
+          s = G[vsw<NP>(xe)];
+        } else {
+          s = G[vsw<NP>(x0)] * Lv[0];
+#pragma unroll
+          for (int l = 1; l < n; ++l) s = s + G[vsw<NP>(x0 + l * xs)] * Lv[l];
+        }
+        if (L.br2) s = s + jump * fg[d * n2];
+        gf[(d * 5 + v) * n2] = s;
       }
-      if (L.br2) {
-        const int d = c / 5, v = c - 5 * d;
-        s = s + bw * (ps[liftc[v] * n2] - pm[liftc[v] * n2]) * fg[d * n2];
-      }
-      gf[c * n2] = s;
     }
   }
 }

@@ -33,8 +33,10 @@ template <typename R, int SPL, int PAR> constexpr size_t volume_smem() {
   return sizeof(R) * (size_t)EPB * (gx::vol_stage_slots<NP, R>(SPL, PAR) + (SPL >= 0 ? 15 * gx::vol_line_threads<NP, R>() : 0)) *
          NP * NP * NP;
 }
-template <typename R> constexpr size_t lift_smem() {
-  return sizeof(R) * (size_t)EPB * (gx::lift_ps_slots(NP) + 15 * NP * NP * NP);
+// faces: the surface flux vectors of all six faces in the FP32 form (not for Gauss-Lobatto BR1)
+template <typename R> constexpr size_t lift_smem(bool faces = true) {
+  return sizeof(R) * (size_t)EPB *
+         (gx::lift_ps_slots(NP) + 15 * NP * NP * NP + (faces && gx::lift_all_faces<NP, R>() ? 90 * NP * NP : 0));
 }
 
 // opt-in shared memory per block of the current device (227 KB on GB300)
@@ -237,7 +239,7 @@ void rhs_front(dg_ctx* ctx, PrecData<R>& P, const S* U, const gx::Gas<R>& gas, c
       }
     }
     if (!lines)
-      gx::k_lift<NP, R, V0><<<grid, NT, lift_smem<R>(), st>>>(P.Pvol.p, P.Met.p, P.Pf.p, P.Fgeo.p, ctx->E2S.p, b, L,
+      gx::k_lift<NP, R, V0><<<grid, NT, lift_smem<R>(L.gauss || L.br2), st>>>(P.Pvol.p, P.Met.p, P.Pf.p, P.Fgeo.p, ctx->E2S.p, b, L,
                                                               P.Gvol.p, P.Gf.p);
     ctx->launches++;
   }
