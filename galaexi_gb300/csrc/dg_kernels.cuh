@@ -9,7 +9,8 @@
 // (k_lift is skipped for the Euler equations; a solution filter adds k_filter / k_filter_laf in front,
 // meshes with boundary sides add k_bc_lift_ghost before k_lift and k_bc_face beside k_face.)  The
 // reference runs ~25-35 launches per stage with full-size intermediates; here the element's state
-// lives in shared memory inside each phase.
+// lives in shared memory inside each phase.  The FP64 form has lifting, face and volume kernels of its own for
+// most configurations (dg_lift_fx.cuh, dg_lift_gfx.cuh, dg_face_fx.cuh, dg_volume_fx.cuh, dg_volume_wfx.cuh).
 //
 // Layouts (internal, all per element contiguous so that element blocks load coalesced):
 //   Pvol [e][7][n^3]     rho,u,v,w,p,T,1/rho                 (compute type R)
