@@ -134,15 +134,16 @@ __host__ __device__ constexpr int lift_ps_slots(int NP) { return 5 * NP * NP * N
 template <int NP, typename R> __host__ __device__ constexpr bool lift_all_faces() { return sizeof(R) == 4 && NP >= 3 && NP <= 9; }
 
 // =====================================================================================
-// k_prolong: ConsToPrim_Volume + ProlongToFace_CUDA + GetPrimitiveStateSurface.  At least two
-// blocks per SM for the FP64 form (FP64-issue bound); three for the mixed form up to N = 7, whose FP64
+// k_prolong: ConsToPrim_Volume + ProlongToFace_CUDA + GetPrimitiveStateSurface.  Three blocks
+// per SM up to N = 7: with two, latency left the FP64 pipe of the FP64 form at 54% (N = 7); the mixed form's FP64
 // work is only E - ke and p - p_ref once its conversions run on the integer pipes (latency bound).
 // =====================================================================================
 template <int NP, typename R> struct ProlongMinBlocks {
-  // three blocks per SM where they fit the SM's 2048 threads (the mixed form up to N = 7), else two;
-  // the mixed form's element of 216 threads (N = 5) five
+  // three blocks per SM where they fit the SM's 2048 threads (up to N = 7), else two; the mixed form's element of
+  // 216 threads (N = 5) five.  FP64 form with three instead of two: N = 7, 24^3 0.300 -> 0.233 ms, N = 6, 27^3
+  // 0.378 -> 0.287, Gauss N = 7, 20^3 0.456 -> 0.413; the other degrees have more blocks either way
   static constexpr int v =
-      (OffsetOf<R>::v && NP == 6) ? 5 : ((OffsetOf<R>::v && 3 * EPBof<NP>::v * NP * NP * NP <= 2048) ? 3 : 2);
+      (OffsetOf<R>::v && NP == 6) ? 5 : (((OffsetOf<R>::v || sizeof(R) == 8) && 3 * EPBof<NP>::v * NP * NP * NP <= 2048) ? 3 : 2);
 };
 // threads of a block of EPB elements: one per node; a single small element (of a mesh that leaves SMs without a
 // block at EPBof elements per block) one per face node too
