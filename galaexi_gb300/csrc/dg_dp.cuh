@@ -24,40 +24,56 @@ __device__ __forceinline__ double dp_widen(float f, int k) {
   const int b = __float_as_int(f);
   return __hiloint2double((((b >> 23) + 1023 - 127 + k) << 20) | ((b & 0x7fffff) >> 3), b << 29);
 }
+// Outside the exponents for which the FP32 approximations and the remainders below are normal numbers (zeros,
+// subnormal and huge numbers, infinities, NaN) the helpers return what CUDA's operators return.
 static __device__ __noinline__ double dp_rcp_rare(double x) { return 1. / x; }
 static __device__ __noinline__ double dp_div_rare(double a, double b) { return a / b; }
 static __device__ __noinline__ double dp_rsqrt_rare(double x) { return 1. / sqrt(x); }
+static __device__ __noinline__ double dp_sqrt_rare(double x) { return sqrt(x); }
+// biased exponent e0 .. e0 + count - 1 (sign aside)
+__device__ __forceinline__ bool dp_exponent_in(double x, int e0, int count) {
+  return (unsigned)(((__double2hiint(x) >> 20) & 0x7ff) - e0) < (unsigned)count;
+}
 
-// 1/x: Newton-Raphson r <- r + r (1 - x r) from the 22-bit FP32 approximation of the mantissa's reciprocal
+// 1/x: Newton-Raphson r <- r + r (1 - x r) from the 22-bit FP32 approximation of the mantissa's reciprocal.  The
+// last step's correction is exact to 2^-33 ulp, so the result is the rounded quotient or, next to a tie, its
+// neighbour.
 __device__ __forceinline__ double dp_rcp(double x) {
   const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
-  if ((unsigned)(e - 123) >= 1800u) return dp_rcp_rare(x);  // zero, subnormal, huge, infinite, NaN
+  if (!dp_exponent_in(x, 123, 1800)) return dp_rcp_rare(x);
   const float m = __int_as_float(0x3f800000 | ((hi & 0xfffff) << 3) | (int)((unsigned)__double2loint(x) >> 29));
   double r = dp_widen(__fdividef(1.f, m), 1023 - e);
   r = __hiloint2double(__double2hiint(r) | (hi & 0x80000000), __double2loint(r));
   r = fma(r, fma(-x, r, 1.), r);
   return fma(r, fma(-x, r, 1.), r);
 }
-// a/b with the remainder of the first quotient
+// a/b with the remainder of the first quotient (as close to the rounded quotient as dp_rcp); both within
+// 2^-500 .. 2^500, where quotient and remainder are normal numbers
 __device__ __forceinline__ double dp_div(double a, double b) {
-  if ((unsigned)(((__double2hiint(b) >> 20) & 0x7ff) - 123) >= 1800u) return dp_div_rare(a, b);
+  if (!dp_exponent_in(a, 523, 1000) || !dp_exponent_in(b, 523, 1000)) return dp_div_rare(a, b);
   const double r = dp_rcp(b), q = a * r;
   return fma(fma(-b, q, a), r, q);
 }
-// 1/sqrt(x) for x > 0: Newton's iteration y <- y + y/2 (1 - x y y) from the FP32 approximation
-__device__ __forceinline__ double dp_rsqrt(double x) {
+// y = 1/sqrt(x) by Newton's iteration y <- y + y/2 (1 - x y y) from the FP32 approximation, to one ulp (the rounding
+// of x y), and sqrt(x): with the remainder of x y (EXACT) or x y itself, to two ulp
+template <bool EXACT>
+__device__ __forceinline__ double dp_root(double x, double& y) {
   const int hi = __double2hiint(x);
-  if ((unsigned)((hi >> 20) - 123) >= 1800u) return dp_rsqrt_rare(x);  // also every negative x
+  if ((unsigned)((hi >> 20) - 123) >= 1800u) {  // also every negative x
+    y = dp_rsqrt_rare(x);
+    return dp_sqrt_rare(x);
+  }
   const int e = (hi >> 20) - 1023, k = e >> 1;  // x = m 2^(2k), 1 <= m < 4
   const float m = __int_as_float(((127 + (e - 2 * k)) << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)__double2loint(x) >> 29));
-  double y = dp_widen(rsqrtf(m), -k);
+  y = dp_widen(rsqrtf(m), -k);
   y = fma(dp_scale(y, -1), fma(-(x * y), y, 1.), y);
-  return fma(dp_scale(y, -1), fma(-(x * y), y, 1.), y);
-}
-// sqrt(x) from y = 1/sqrt(x), with the remainder of x y
-__device__ __forceinline__ double dp_sqrt_from(double x, double y) {
+  y = fma(dp_scale(y, -1), fma(-(x * y), y, 1.), y);
   const double s = x * y;
-  return fma(fma(-s, s, x), dp_scale(y, -1), s);
+  return EXACT ? fma(fma(-s, s, x), dp_scale(y, -1), s) : s;
+}
+__device__ __forceinline__ double dp_sqrt(double x) {
+  double y;
+  return dp_root<true>(x, y);
 }
 
 }  // namespace gx

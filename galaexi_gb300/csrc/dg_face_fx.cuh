@@ -59,7 +59,7 @@ __device__ __forceinline__ void riemann_dp(const double dm[3], const FaceSide& L
     central_flux<CENTRAL>(L, R, n, HL, HR, F);
     // |u_n| + c: the larger temperature has the larger sound speed
     const double c2 = g.kR * dp_max(L.T, R.T);
-    const double hl = 0.5 * (dp_max(dp_abs(L.un), dp_abs(R.un)) + dp_sqrt_from(c2, dp_rsqrt(c2)));
+    const double hl = 0.5 * (dp_max(dp_abs(L.un), dp_abs(R.un)) + dp_sqrt(c2));
     F[0] = F[0] - hl * (R.rho - L.rho);
 #pragma unroll
     for (int c = 0; c < 3; ++c) F[1 + c] = F[1 + c] - hl * dm[c];
@@ -70,7 +70,7 @@ __device__ __forceinline__ void riemann_dp(const double dm[3], const FaceSide& L
   double rr = L.rho * R.rho;
   // (two negative densities: no square root)
   rr = __hiloint2double(__double2hiint(rr) | (__double2hiint(L.rho) & (int)0x80000000), __double2loint(rr));
-  const double rt = dp_sqrt_from(rr, dp_rsqrt(rr));
+  const double rt = dp_sqrt(rr);
   const double w = R.rho * dp_rcp(R.rho + rt);
   const double un = fma(w, R.un - L.un, L.un);
   double u[3];
@@ -78,7 +78,9 @@ __device__ __forceinline__ void riemann_dp(const double dm[3], const FaceSide& L
   for (int c = 0; c < 3; ++c) u[c] = fma(w, R.v[c] - L.v[c], L.v[c]);
   const double H = fma(w, HR - HL, HL);
   const double q2 = 0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
-  const double c2 = g.kappaM1 * (H - q2), ic = dp_rsqrt(c2), c = c2 * ic;
+  const double c2 = g.kappaM1 * (H - q2);
+  double ic;
+  const double c = dp_root<false>(c2, ic);
   if constexpr (RIEM == DG_RIEMANN_HLLC) {
     const double Sl = un - c, Sr = un + c;
     const double mnL = L.rho * (Sl - L.un), mnR = R.rho * (Sr - R.un);
@@ -104,7 +106,7 @@ __device__ __forceinline__ void riemann_dp(const double dm[3], const FaceSide& L
   double l1 = un - c, l2 = un, l5 = un + c;
   if constexpr (RIEM == DG_RIEMANN_ROEENTROPYFIX) {
     const double aL = g.kR * L.T, aR = g.kR * R.T;
-    const double cL = dp_sqrt_from(aL, dp_rsqrt(aL)), cR = dp_sqrt_from(aR, dp_rsqrt(aR));
+    const double cL = dp_sqrt(aL), cR = dp_sqrt(aR);
     auto fix = [](double a, double al, double ar) {
       const double da = dp_max(dp_max(a - al, ar - a), 0.), ab = dp_abs(a);
       return dp_bits(ab) < dp_bits(da) ? 0.5 * (dp_div(a * a, da) + da) : ab;
