@@ -77,6 +77,13 @@ void weak_basis(const dg_ctx* ctx, gx::VolWfxBasis<NP>& wb) {
   all = Dh;
   all.insert(all.end(), Lh.begin(), Lh.end());
   wb.sD = 60 - exponent(all);
+  double most = 0.;
+  for (int i = 0; i < NP; ++i) {
+    double sum = std::fabs(Lh[i].h) + std::fabs(Lh[N - i].h);
+    for (int l = 0; l < NP; ++l) sum += std::fabs(Dh[i * NP + l].h);
+    most = std::fmax(most, sum);
+  }
+  wb.S = (int)std::floor(63. - std::log2(3. * most) - 1e-3 - (59 + wb.sD - 64));
   auto half = [](gxh::DD a) { return gxh::dd_mul(a, gxh::dd_num(0.5)); };
   auto at = [&](int i, int l) { return Dh[i * NP + l]; };
   for (int i = 0; i < HE; ++i) {

@@ -34,7 +34,7 @@ template <int NP> struct VolWfx {
 template <int NP> struct VolWfxBasis {
   static constexpr int H = NP / 2, HE = (NP + 1) / 2;
   FxLimb even[H][HE], odd[HE][H], lo[H], le[HE];
-  int sD;
+  int sD, S;  // S: shift of the contractions, 3 * 2^59 * (largest row sum of |D_hat|, |L_hat|) * 2^(sD - 64 + S) < 2^63
 };
 // one direction: metric terms * 2^sM, left shifts of the products, right shifts of M.m, scales of the rows' fluxes;
 // the stresses' scales
@@ -49,9 +49,10 @@ struct VolWfxScale {
 enum { W_M2, W_U2, W_P, W_E, W_TAU, W_TQ, W_F, W_V = W_F + 15, W_NMAX, W_PMIN = W_NMAX, W_N };
 
 // Scales of one element, by the first warp (lanes 0-2: one direction each).  Rows, with Mm = M_d.m (m = rho u): mass
-// Mm, momentum c: Mm v_c + M_d,c p - M_d.tau_c, energy Mm (E+p)/rho - M_d.tq; each below 2^57 at its scale 2^t, the
-// face fluxes too, so that a line's contraction (|D_hat| < 2^60, at most five even and five odd products of sums of
-// two, and two face terms) stays below 2^60 after its shift by 4, and the sum of three directions below 2^62.
+// Mm, momentum c: Mm v_c + M_d,c p - M_d.tau_c, energy Mm (E+p)/rho - M_d.tq; each below 2^59 at its scale 2^t, the
+// face fluxes too, so that the mixed products of a line's contraction (limbs of |D_hat| < 2^60, at most five products
+// of sums of two and one face term) stay below 2^63; the contraction is shifted by as much as the rows of D_hat and
+// L_hat allow (VolWfxBasis::S), so that the sum of three directions stays below 2^63.
 // p, the stresses and (E+p)/rho have one scale each for the three directions, and the products of a direction's
 // row are shifted to it at the end; Mm is shifted to the scale of M p before its product with v.
 template <int PARAB>
@@ -73,18 +74,18 @@ __device__ __forceinline__ void vol_wfx_scales(const unsigned* mag, const float*
   const int s_m = 59 - ((int)floorf(Lm) + 1), s_v = 59 - ((int)floorf(Lu) + 1);
   const int sV = (int)floorf(60.4f - LV);
   o.hV = sV - (o.sM + s_m - 64);
-  o.t[0] = (int)floorf(56.9f - fmaxf(LV, fx_log2(mag[W_F + 5 * d])));
+  o.t[0] = (int)floorf(58.9f - fmaxf(LV, fx_log2(mag[W_F + 5 * d])));
   o.k0 = min(sV - o.t[0], 63);
   // scales of the momentum and energy rows
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     float L = fx_lse(LV + Lu, (ok ? MetL[3 + 3 * d + c] : 0.f) + Lp);
     if (PARAB) L = fx_lse(L, LM + Lt);
-    o.t[1 + c] = (int)floorf(56.9f - fmaxf(L, fx_log2(mag[W_F + 5 * d + 1 + c])));
+    o.t[1 + c] = (int)floorf(58.9f - fmaxf(L, fx_log2(mag[W_F + 5 * d + 1 + c])));
   }
   float Le = LV + LE;
   if (PARAB) Le = fx_lse(Le, LM + Lq);
-  o.t[4] = (int)floorf(56.9f - fmaxf(Le, fx_log2(mag[W_F + 5 * d + 4])));
+  o.t[4] = (int)floorf(58.9f - fmaxf(Le, fx_log2(mag[W_F + 5 * d + 4])));
   // p and the stresses: below 2^60, M p no finer than Mm v can be, and not finer than the rows' scales; tq in the
   // same way beside Mm (E+p)/rho
   const int s_E = 60 - fx_exp(mag[W_E]);
@@ -323,12 +324,12 @@ k_volume_wfx(const double* __restrict__ U, const double* __restrict__ Pvol, cons
         fx64 mB = fx_mid(fs, wb.le[i], 0), hB = fx_mad(fs.h, wb.le[i].h, 0);
 #pragma unroll
         for (int l = 0; l < H; ++l) { mB = fx_mid(od[l], wb.odd[i][l], mB); hB = fx_mad(od[l].h, wb.odd[i][l].h, hB); }
-        const fx64 B = fx_shift(hB + (mB >> 32), mB, 4);
+        const fx64 B = fx_shift(hB + (mB >> 32), mB, wb.S);
         if (i < H) {
           fx64 mA = fx_mid(fd, wb.lo[i], 0), hA = fx_mad(fd.h, wb.lo[i].h, 0);
 #pragma unroll
           for (int l = 0; l < HE; ++l) { mA = fx_mid(ev[l], wb.even[i][l], mA); hA = fx_mad(ev[l].h, wb.even[i][l].h, hA); }
-          const fx64 a = fx_shift(hA + (mA >> 32), mA, 4);
+          const fx64 a = fx_shift(hA + (mA >> 32), mA, wb.S);
           f[vsw<NP>(base + i * step)] = a + B;
           f[vsw<NP>(base + (N - i) * step)] = B - a;
         } else {
@@ -372,7 +373,7 @@ k_volume_wfx(const double* __restrict__ U, const double* __restrict__ Pvol, cons
         fx64 r = 0;
 #pragma unroll
         for (int d = 0; d < 3; ++d) r += fx_sar(a[(5 * d + v) * n3], min(sc.d[d].t[v] - sc.t[v], 63));
-        const int k = sc.t[v] + wb.sD - 64 + 4;
+        const int k = sc.t[v] + wb.sD - 64 + wb.S;
         ut[v] = __ll2double_rn(r) * __hiloint2double(ch - (k << 20), cl);
       }
     } else {
