@@ -45,8 +45,8 @@ struct VolWfxScale {
   VolWfxDir d[3];
   int s_m, s_v, s_p, s_E, s_t, s_q, t[5], ok;
 };
-// largest magnitudes: W_M2, W_U2 float bits of |m|^2 and |u|^2; W_F: face fluxes [direction][row]
-enum { W_M2, W_U2, W_P, W_E, W_TAU, W_TQ, W_F, W_V = W_F + 15, W_NMAX, W_PMIN = W_NMAX, W_N };
+// largest magnitudes: W_M2, W_U2 float bits of |m|^2 and |u|^2; W_R: 1/rho; W_F: face fluxes [direction][row]
+enum { W_M2, W_U2, W_P, W_E, W_TAU, W_TQ, W_F, W_V = W_F + 15, W_R, W_NMAX, W_PMIN = W_NMAX, W_RMIN, W_N };
 
 // Scales of one element, by the first warp (lanes 0-2: one direction each).  Rows, with Mm = M_d.m (m = rho u): mass
 // Mm, momentum c: Mm v_c + M_d,c p - M_d.tau_c, energy Mm (E+p)/rho - M_d.tq; each below 2^59 at its scale 2^t, the
@@ -55,6 +55,9 @@ enum { W_M2, W_U2, W_P, W_E, W_TAU, W_TQ, W_F, W_V = W_F + 15, W_NMAX, W_PMIN = 
 // L_hat allow (VolWfxBasis::S), so that the sum of three directions stays below 2^63.
 // p, the stresses and (E+p)/rho have one scale each for the three directions, and the products of a direction's
 // row are shifted to it at the end; Mm is shifted to the scale of M p before its product with v.
+// Elements whose densities differ by more than 2^3 to 2^4 take the FP64 sums: at one pressure and velocity, rho u and
+// (E+p)/rho have their maxima at opposite nodes, and the energy row's bound is above its products by the contrast
+// (errors of the worst row, contrasts 8, 16, 64, 256: 0.65, 1.2, 2.4 and 5 times the FP64 kernel's).
 template <int PARAB>
 __device__ __forceinline__ void vol_wfx_scales(const unsigned* mag, const float* MetL, VolWfxScale& S, int lane) {
   const int d = min(lane, 2);
@@ -64,6 +67,7 @@ __device__ __forceinline__ void vol_wfx_scales(const unsigned* mag, const float*
   const unsigned lowest = (1022u - 150u) << 20;
   ok = ok && (mag[W_V] == 0u || mag[W_V] >= (1023u - 60u) << 20);  // the range of fx_float
   ok = ok && mag[W_PMIN] > lowest && mag[W_E] > lowest && (mag[W_P] >> 20) - (mag[W_PMIN] >> 20) <= 8;
+  ok = ok && mag[W_RMIN] > lowest && (mag[W_R] >> 20) - (mag[W_RMIN] >> 20) <= 3;
   const float LM = ok ? MetL[d] : 0.f;
   const float Lm = 0.5f * __log2f(__uint_as_float(mag[W_M2])) + 1e-4f, Lu = 0.5f * __log2f(__uint_as_float(mag[W_U2])) + 1e-4f;
   const float Lp = fx_log2(mag[W_P]), LE = fx_log2(mag[W_E]);
@@ -199,13 +203,15 @@ k_volume_wfx(const double* __restrict__ U, const double* __restrict__ Pvol, cons
   const double* const Ge = PARAB ? Gvol + (size_t)e * 15 * n3 : nullptr;
   // ---- largest magnitudes; (E + p)/rho and the stresses wait in the node's slots as FP64
   {
-    unsigned m[6] = {0u, 0u, 0u, 0u, 0u, 0u}, mV = 0u, pmin = 0xffffffffu;
+    unsigned m[6] = {0u, 0u, 0u, 0u, 0u, 0u}, mV = 0u, pmin = 0xffffffffu, mr = 0u, rmin = 0xffffffffu;
     vol_flux_max<NP, NT>(Flux, es, &mag[W_F]);
 #pragma unroll 1
     for (int node = tid; node < n3; node += NT) {
       const double* P = Pe + node;
       const double vel[3] = {P[n3], P[2 * n3], P[3 * n3]}, p = P[4 * n3];
-      const double Ep = (Ue[node * 5 + 4] + p) * P[6 * n3];
+      const double srho = P[6 * n3], Ep = (Ue[node * 5 + 4] + p) * srho;
+      mr = max(mr, fx_mag(srho));
+      rmin = min(rmin, fx_mag(srho));
       fx64* const a = A + vsw<NP>(node);
       a[0] = __double_as_longlong(Ep);
       auto norm2 = [](double x, double y, double z) {
@@ -237,6 +243,8 @@ k_volume_wfx(const double* __restrict__ U, const double* __restrict__ Pvol, cons
     for (int c = 0; c < (PARAB ? 6 : 4); ++c) fx_block_max(m[c], &mag[c]);
     fx_block_max(mV, &mag[W_V]);
     fx_block_min(pmin, &mag[W_PMIN]);
+    fx_block_max(mr, &mag[W_R]);
+    fx_block_min(rmin, &mag[W_RMIN]);
   }
   __syncthreads();
   if (tid < 32) vol_wfx_scales<PARAB>(mag, MetL + (size_t)e * 16, sc, tid);
