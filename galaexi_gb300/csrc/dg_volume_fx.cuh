@@ -34,7 +34,8 @@ template <int NP> struct VolFx {
   static constexpr int LPW = 32 / TPL;                            // lines per warp
   static constexpr int TPD = (NP * NP + LPW - 1) / LPW;           // warp tasks per direction
   static constexpr int TPW = (OWN == 1 && TPD > 1) || TPD > 16 ? 2 : 1;         // tasks of one warp per direction
-  static constexpr int NW = (TPD + TPW - 1) / TPW, NT = 32 * NW;  // warps and threads of a block
+  // warps and threads of a block (n = 10: one warp more, so that vol_block_fp64's 300 lines have a thread each)
+  static constexpr int NW = NP == 10 ? 10 : (TPD + TPW - 1) / TPW, NT = 32 * NW;
   static constexpr int NPT = (NP * NP * NP + NT - 1) / NT;        // nodes per thread
   // blocks per SM for 128 registers per thread (512 threads), where shared memory holds them
   static constexpr int MINB = NP >= 9 ? 1 : (512 / NT < 16 ? 512 / NT : 16);
@@ -208,67 +209,197 @@ __device__ __forceinline__ void vol_flux_max(const double* Flux, const int* es, 
   }
 }
 
-// The same sums in FP64 for one node, from global memory: for elements whose values do not fit one scale
-// per quantity (infinities and NaN, magnitudes outside 2^+-150, densities or pressures that differ by more
-// than 2^8 within the element, which one scale would hold less exactly than FP64).
-template <int NP, int SPLIT, int PARAB>
-__device__ __noinline__ void vol_node_fp64(const double* U, const double* Pe, const double* Ge, const double* Me,
-                                           const double* Flux, const int* es, const double* DVS, const double* DhatT,
-                                           double Lhm0, double LhpN, const Gas<double>& gas, int node, double ut[5]) {
-  constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP, N = NP - 1;
-  auto load = [&](int x, PairNode<double>& a) {
-    a.rho = Pe[x]; a.u = Pe[n3 + x]; a.v = Pe[2 * n3 + x]; a.w = Pe[3 * n3 + x]; a.pm = Pe[4 * n3 + x];
-    a.m1 = a.m2 = a.m3 = 0.;
-    a.aux = pair_aux<SPLIT, double>(a.rho, a.u, a.v, a.w, U[x * 5 + 4], a.pm, Pe[6 * n3 + x]);
-  };
-  const int ijk[3] = {node % n, (node / n) % n, node / n2};
-  double acc[5] = {0., 0., 0., 0., 0.};
-  PairNode<double> a;
-  load(node, a);
+// The same sums in FP64 by the block, in the operations of k_volume: for elements whose values do not fit one scale
+// per quantity (infinities and NaN, magnitudes outside 2^+-150, densities or pressures that differ by more than the
+// scales allow within the element, which one scale would hold less exactly than FP64).  Bound by the FP64 pipe like
+// k_volume, whose work it does: the viscous or weak fluxes once per node, each pair once.  SPLIT < 0: weak form.
+// A: the block's shared memory, of which the fixed-point values are not needed any more (SPLIT < 0: 15 slots, else
+// 27, or 21 for the Euler equations); the results are left there as [node][5].  D: n^2 words for the split form's
+// matrix (the limbs' place: with words of its own the block of n = 4 fits an SM 14 instead of 15 times).
+template <int NP, int SPLIT, int PARAB, int NT>
+__device__ __noinline__ void vol_block_fp64(const double* U, const double* Pe, const double* Ge, const double* Me,
+                                            const double* Flux, const int* es, DevBasis<double> basis, int gauss,
+                                            double mu, double lambda, double* D, double* A) {
+  constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP, N = NP - 1, NPT = (n3 + NT - 1) / NT;
+  constexpr int v0 = SPLIT < 0 ? 0 : 1, nvs = 5 - v0;  // slots of flux (d, v): d nvs + v - v0
+  const int tid = threadIdx.x;
+  double acc[NPT][5];
+#pragma unroll
+  for (int it = 0; it < NPT; ++it)
+#pragma unroll
+    for (int v = 0; v < 5; ++v) acc[it][v] = 0.;
+  __syncthreads();
+  if constexpr (SPLIT < 0 || PARAB) {
 #pragma unroll 1
-  for (int dir = 0; dir < 3; ++dir) {
-    const int step = dir == 0 ? 1 : (dir == 1 ? n : n2), i = ijk[dir], base = node - i * step;
-    const double* M = Me + (size_t)3 * dir * n3;
-#pragma unroll 1
-    for (int l = 0; l < n; ++l) {
-      const int x = base + l * step;
-      PairNode<double> b;
-      load(x, b);
-      if (l != i) {
-        double F[5];
-        split_pair_flux<SPLIT, double>(a, b, M[node] + M[x], M[n3 + node] + M[n3 + x], M[2 * n3 + node] + M[2 * n3 + x],
-                                       0., F);
-        for (int v = 0; v < 5; ++v) acc[v] = acc[v] + DVS[l + n * i] * F[v];
-      }
+    for (int node = tid; node < n3; node += NT) {
+      const double* const P = Pe + node;
+      const double vel[3] = {P[n3], P[2 * n3], P[3 * n3]};
+      double tau[6] = {0., 0., 0., 0., 0., 0.}, tq[3] = {0., 0., 0.};
       if constexpr (PARAB) {
-        double g[15], tau[6], tq[3];
-        for (int c = 0; c < 15; ++c) g[c] = c % 5 ? Ge[c * n3 + x] : 0.;
-        const double vel[3] = {b.u, b.v, b.w};
-        visc_stress(g, g + 5, g + 10, vel, gas.mu, gas.lambda, tau, tq);
-        const double m0 = M[x], m1 = M[n3 + x], m2 = M[2 * n3 + x], d = DhatT[l + n * i];
-        acc[1] = acc[1] + d * (-m0 * tau[0] - m1 * tau[3] - m2 * tau[4]);
-        acc[2] = acc[2] + d * (-m0 * tau[3] - m1 * tau[1] - m2 * tau[5]);
-        acc[3] = acc[3] + d * (-m0 * tau[4] - m1 * tau[5] - m2 * tau[2]);
-        acc[4] = acc[4] + d * (-m0 * tq[0] - m1 * tq[1] - m2 * tq[2]);
+        const double* const G = Ge + node;
+        const double gx[5] = {0., G[n3], G[2 * n3], G[3 * n3], G[4 * n3]};
+        const double gy[5] = {0., G[6 * n3], G[7 * n3], G[8 * n3], G[9 * n3]};
+        const double gz[5] = {0., G[11 * n3], G[12 * n3], G[13 * n3], G[14 * n3]};
+        visc_stress(gx, gy, gz, vel, mu, lambda, tau, tq);
+      }
+      const double *const Un = U + node * 5, p = P[4 * n3], Ep = SPLIT < 0 ? (Un[4] + p) * P[6 * n3] : 0.;
+      double* const a = A + vsw<NP>(node);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const double m0 = Me[3 * d * n3 + node], m1 = Me[(3 * d + 1) * n3 + node], m2 = Me[(3 * d + 2) * n3 + node];
+        double f[5] = {0., 0., 0., 0., 0.};
+        if constexpr (SPLIT < 0) {
+          const double mm = m0 * Un[1] + m1 * Un[2] + m2 * Un[3];
+          f[0] = mm;
+          f[1] = mm * vel[0] + m0 * p;
+          f[2] = mm * vel[1] + m1 * p;
+          f[3] = mm * vel[2] + m2 * p;
+          f[4] = mm * Ep;
+        }
+        if constexpr (PARAB) {
+          f[1] = f[1] - m0 * tau[0] - m1 * tau[3] - m2 * tau[4];
+          f[2] = f[2] - m0 * tau[3] - m1 * tau[1] - m2 * tau[5];
+          f[3] = f[3] - m0 * tau[4] - m1 * tau[5] - m2 * tau[2];
+          f[4] = f[4] - m0 * tq[0] - m1 * tq[1] - m2 * tq[2];
+        }
+#pragma unroll
+        for (int v = v0; v < 5; ++v) a[(d * nvs + v - v0) * n3] = f[v];
       }
     }
-  }
-#pragma unroll 1
-  for (int ls = 1; ls <= 6; ++ls) {
-    const int dir = ls == L_XI_MINUS || ls == L_XI_PLUS ? 0 : (ls == L_ETA_MINUS || ls == L_ETA_PLUS ? 1 : 2);
-    if (ijk[dir] != (is_minus(ls) ? 0 : N)) continue;
-    const int fa = dir == 0 ? ijk[1] : ijk[0], fb = dir == 2 ? ijk[1] : ijk[2];
-    const int side = es[2 * (ls - 1)], flip = es[2 * (ls - 1) + 1];
-    int p, q;
-    s2v2_inv(N, fa, fb, flip, ls, p, q);
-    const double Lh = is_minus(ls) ? Lhm0 : LhpN;
-    for (int v = 0; v < 5; ++v) {
-      const double f = Flux[((size_t)side * 5 + v) * n2 + p + n * q];
-      acc[v] = acc[v] + (flip == 0 ? f : -f) * Lh;
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < NPT; ++it) {
+      const int node = tid + it * NT;
+      if (node >= n3) break;
+      const int i = node % n, j = (node / n) % n, k = node / n2;
+#pragma unroll 4
+      for (int l = 0; l < n; ++l) {
+        const double ci = basis.DhatT[l + n * i], cj = basis.DhatT[l + n * j], ck = basis.DhatT[l + n * k];
+        const int ni = vsw<NP>(l + n * (j + n * k)), nj = vsw<NP>(i + n * (l + n * k)), nk = vsw<NP>(i + n * (j + n * l));
+#pragma unroll
+        for (int v = v0; v < 5; ++v)
+          acc[it][v] = acc[it][v] + ci * A[(v - v0) * n3 + ni] + ck * A[(2 * nvs + v - v0) * n3 + nk] +
+                       cj * A[(nvs + v - v0) * n3 + nj];
+      }
     }
+    __syncthreads();
   }
-  const double sj = Me[(size_t)9 * n3 + node];
-  for (int v = 0; v < 5; ++v) ut[v] = acc[v] * -1. * sj;
+  if constexpr (SPLIT >= 0) {
+    // one thread per line, node b's share of a pair (a, b) to the line's own sums in shared memory
+    double* const S = A + (PARAB ? 12 : 6) * n3;  // [3][5][n3]
+    for (int t = tid; t < n2; t += NT) D[t] = SPLIT == DG_SPLIT_PI ? dp_scale(basis.DVS[t], -3) : basis.DVS[t];
+#pragma unroll 1
+    for (int node = tid; node < n3; node += NT) {
+      const double* const P = Pe + node;
+      double* const a = A + vsw<NP>(node);
+      const double rho = P[0], u = P[n3], v = P[2 * n3], w = P[3 * n3], p = P[4 * n3];
+      a[0] = rho; a[2 * n3] = u; a[3 * n3] = v; a[4 * n3] = w; a[5 * n3] = SPLIT == DG_SPLIT_PI ? 4. * p : p;
+      a[n3] = pair_aux<SPLIT, double>(rho, u, v, w, U[node * 5 + 4], p, P[6 * n3]);
+      for (int c = 0; c < 15; ++c) S[c * n3 + vsw<NP>(node)] = 0.;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int t = tid; t < 3 * n2; t += NT) {
+      const int dir = t / n2, li = t - dir * n2, step = dir == 0 ? 1 : (dir == 1 ? n : n2);
+      const int base = dir == 0 ? n * li : (dir == 1 ? (li % n) + n2 * (li / n) : li);
+      double* const Sd = S + dir * 5 * n3;
+      const double* const M = Me + 3 * dir * n3;
+      auto load = [&](int s, PairNode<double>& x) {
+        x.rho = A[s]; x.aux = A[n3 + s]; x.u = A[2 * n3 + s]; x.v = A[3 * n3 + s]; x.w = A[4 * n3 + s]; x.pm = A[5 * n3 + s];
+        x.m1 = x.m2 = x.m3 = 0.;
+      };
+#pragma unroll 1
+      for (int ia = 0; ia < n - 1; ++ia) {
+        const int na = base + ia * step, sa = vsw<NP>(na);
+        PairNode<double> a;
+        load(sa, a);
+        const double a0 = M[na], a1 = M[n3 + na], a2 = M[2 * n3 + na];
+        double sum[5];
+#pragma unroll
+        for (int v = 0; v < 5; ++v) sum[v] = Sd[v * n3 + sa];
+#pragma unroll 2
+        for (int ib = ia + 1; ib < n; ++ib) {
+          const int nb = base + ib * step, sb = vsw<NP>(nb);
+          PairNode<double> b;
+          load(sb, b);
+          double F[5];
+          const double M0 = a0 + M[nb], M1 = a1 + M[n3 + nb], M2 = a2 + M[2 * n3 + nb];
+          if constexpr (SPLIT == DG_SPLIT_PI) {
+            // 8 F, the density row 4 F, and DVolSurf / 8 (exact scalings)
+            const double us = a.u + b.u, vs = a.v + b.v, ws = a.w + b.w, ps = a.pm + b.pm;
+            const double q = (a.rho + b.rho) * (M0 * us + M1 * vs + M2 * ws);
+            F[0] = q;
+            F[1] = q * us + ps * M0;
+            F[2] = q * vs + ps * M1;
+            F[3] = q * ws + ps * M2;
+            F[4] = q * (a.aux + b.aux);
+          } else {
+            split_pair_flux<SPLIT, double>(a, b, M0, M1, M2, 0., F);
+          }
+          const double dba = D[ib + n * ia], dab = D[ia + n * ib];
+#pragma unroll
+          for (int v = 0; v < 5; ++v) {
+            sum[v] = sum[v] + dba * F[v];
+            Sd[v * n3 + sb] += dab * F[v];
+          }
+        }
+#pragma unroll
+        for (int v = 0; v < 5; ++v) Sd[v * n3 + sa] = sum[v];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < NPT; ++it) {
+      const int node = tid + it * NT, s = vsw<NP>(node);
+      if (node < n3)
+#pragma unroll
+        for (int v = 0; v < 5; ++v) {
+          double x = S[v * n3 + s] + S[(5 + v) * n3 + s] + S[(10 + v) * n3 + s];
+          if (SPLIT == DG_SPLIT_PI && v == 0) x = x * 2.;
+          acc[it][v] = acc[it][v] + x;
+        }
+    }
+    __syncthreads();
+  }
+  // the fluxes of the six faces (slave sides negated), then of each node's lines
+#pragma unroll 1
+  for (int t = tid; t < 6 * n2; t += NT) {
+    const int ls = t / n2 + 1, ab = t - (ls - 1) * n2, side = es[2 * (ls - 1)], flip = es[2 * (ls - 1) + 1];
+    int p, q;
+    s2v2_inv(N, ab % n, ab / n, flip, ls, p, q);
+    const double* const f = Flux + (size_t)side * 5 * n2 + p + n * q;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) A[((ls - 1) * 5 + v) * n2 + ab] = flip == 0 ? f[v * n2] : -f[v * n2];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < NPT; ++it) {
+    const int node = tid + it * NT;
+    if (node >= n3) break;
+    const int i = node % n, j = (node / n) % n, k = node / n2;
+    double ut[5] = {0., 0., 0., 0., 0.};
+#pragma unroll 1
+    for (int ls = 1; ls <= 6; ++ls) {
+      const int dir = ls == L_XI_MINUS || ls == L_XI_PLUS ? 0 : (ls == L_ETA_MINUS || ls == L_ETA_PLUS ? 1 : 2);
+      const int l = dir == 0 ? i : (dir == 1 ? j : k);
+      if (!gauss && l != (is_minus(ls) ? 0 : N)) continue;
+      const double Lh = is_minus(ls) ? basis.Lhm[l] : basis.Lhp[l];
+      const double* const f = A + (ls - 1) * 5 * n2 + (dir == 0 ? j : i) + n * (dir == 2 ? j : k);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) ut[v] = ut[v] + f[v * n2] * Lh;
+    }
+    const double sj = Me[9 * n3 + node];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) acc[it][v] = (acc[it][v] + ut[v]) * -1. * sj;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < NPT; ++it) {
+    const int node = tid + it * NT;
+    if (node < n3)
+#pragma unroll
+      for (int v = 0; v < 5; ++v) A[node * 5 + v] = acc[it][v];
+  }
 }
 
 template <int NP, int SPLIT, int PARAB>
@@ -283,7 +414,7 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
   constexpr int S_RHO = 0, S_AUX = 1, S_VEL = 2, S_P = 5;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   fx64* const A = reinterpret_cast<fx64*>(smem_raw);
-  __shared__ VolFxBasis<NP> sb;
+  __shared__ __align__(8) VolFxBasis<NP> sb;
   __shared__ unsigned mag[X_N];
   __shared__ VolFxScale sc;
   __shared__ int es[12];
@@ -603,13 +734,8 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
       }
     }
   } else {
-    for (int node = tid; node < n3; node += NT) {
-      double ut[5];
-      vol_node_fp64<NP, SPLIT, PARAB>(Ue, Pe, Ge, Me, Flux, es, basis.DVS, basis.DhatT, basis.Lhm[0], basis.Lhp[N], gas,
-                                      node, ut);
-#pragma unroll
-      for (int v = 0; v < 5; ++v) Us[node * 5 + v] = ut[v];
-    }
+    vol_block_fp64<NP, SPLIT, PARAB, NT>(Ue, Pe, Ge, Me, Flux, es, basis, 0, gas.mu, gas.lambda,
+                                         reinterpret_cast<double*>(sb.Q), Us);
   }
   __syncthreads();
   // output / LSERK-W2 stage, one value per thread in turn (the element's record is contiguous)

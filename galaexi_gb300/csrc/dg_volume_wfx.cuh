@@ -129,56 +129,6 @@ __device__ __forceinline__ void vol_wfx_scales(const unsigned* mag, const float*
   }
 }
 
-// the same sums in FP64 for one node, from global memory (elements that do not fit one scale)
-template <int NP, int PARAB>
-__device__ __noinline__ void vol_weak_node_fp64(const double* U, const double* Pe, const double* Ge, const double* Me,
-                                                const double* Flux, const int* es, const double* DhatT, const double* Lhm,
-                                                const double* Lhp, int gauss, const Gas<double>& gas, int node, double ut[5]) {
-  constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP, N = NP - 1;
-  const int ijk[3] = {node % n, (node / n) % n, node / n2};
-  double acc[5] = {0., 0., 0., 0., 0.};
-#pragma unroll 1
-  for (int dir = 0; dir < 3; ++dir) {
-    const int step = dir == 0 ? 1 : (dir == 1 ? n : n2), i = ijk[dir], base = node - i * step;
-#pragma unroll 1
-    for (int l = 0; l < n; ++l) {
-      const int x = base + l * step;
-      const double m0 = Me[(size_t)(3 * dir) * n3 + x], m1 = Me[(size_t)(3 * dir + 1) * n3 + x],
-                   m2 = Me[(size_t)(3 * dir + 2) * n3 + x];
-      const double vel[3] = {Pe[n3 + x], Pe[2 * n3 + x], Pe[3 * n3 + x]}, p = Pe[4 * n3 + x];
-      const double mm = m0 * U[x * 5 + 1] + m1 * U[x * 5 + 2] + m2 * U[x * 5 + 3];
-      double f[5] = {mm, mm * vel[0] + m0 * p, mm * vel[1] + m1 * p, mm * vel[2] + m2 * p,
-                     mm * ((U[x * 5 + 4] + p) * Pe[6 * n3 + x])};
-      if constexpr (PARAB) {
-        double g[15], tau[6], tq[3];
-        for (int c = 0; c < 15; ++c) g[c] = c % 5 ? Ge[(size_t)c * n3 + x] : 0.;
-        visc_stress(g, g + 5, g + 10, vel, gas.mu, gas.lambda, tau, tq);
-        f[1] = f[1] - m0 * tau[0] - m1 * tau[3] - m2 * tau[4];
-        f[2] = f[2] - m0 * tau[3] - m1 * tau[1] - m2 * tau[5];
-        f[3] = f[3] - m0 * tau[4] - m1 * tau[5] - m2 * tau[2];
-        f[4] = f[4] - m0 * tq[0] - m1 * tq[1] - m2 * tq[2];
-      }
-      for (int v = 0; v < 5; ++v) acc[v] = acc[v] + DhatT[l + n * i] * f[v];
-    }
-    for (int pm = 0; pm < 2; ++pm) {
-      if (!gauss && i != (pm == 0 ? 0 : N)) continue;
-      const int ls = dir == 0 ? (pm == 0 ? L_XI_MINUS : L_XI_PLUS)
-                              : (dir == 1 ? (pm == 0 ? L_ETA_MINUS : L_ETA_PLUS) : (pm == 0 ? L_ZETA_MINUS : L_ZETA_PLUS));
-      const int fa = dir == 0 ? ijk[1] : ijk[0], fb = dir == 2 ? ijk[1] : ijk[2];
-      const int side = es[2 * (ls - 1)], flip = es[2 * (ls - 1) + 1];
-      int p, q;
-      s2v2_inv(N, fa, fb, flip, ls, p, q);
-      const double Lh = pm == 0 ? Lhm[i] : Lhp[i];
-      for (int v = 0; v < 5; ++v) {
-        const double f = Flux[((size_t)side * 5 + v) * n2 + p + n * q];
-        acc[v] = acc[v] + (flip == 0 ? f : -f) * Lh;
-      }
-    }
-  }
-  const double sj = Me[(size_t)9 * n3 + node];
-  for (int v = 0; v < 5; ++v) ut[v] = acc[v] * -1. * sj;
-}
-
 template <int NP, int PARAB>
 __global__ void __launch_bounds__(VolWfx<NP>::NT, VolWfx<NP>::MINB)
 k_volume_wfx(const double* __restrict__ U, const double* __restrict__ Pvol, const double* __restrict__ Gvol,
@@ -346,16 +296,9 @@ k_volume_wfx(const double* __restrict__ U, const double* __restrict__ Pvol, cons
       }
     }
     __syncthreads();
-  }
-  else {
-    // (all nodes before any is written: they read their lines' state)
-#pragma unroll 1
-    for (int node = tid; node < n3; node += NT) {
-      double ut[5];
-      vol_weak_node_fp64<NP, PARAB>(Ue, Pe, Ge, Me, Flux, es, basis.DhatT, basis.Lhm, basis.Lhp, gauss, gas, node, ut);
-#pragma unroll
-      for (int v = 0; v < 5; ++v) A[v * n3 + vsw<NP>(node)] = __double_as_longlong(ut[v]);
-    }
+  } else {
+    vol_block_fp64<NP, -1, PARAB, NT>(Ue, Pe, Ge, Me, Flux, es, basis, gauss, gas.mu, gas.lambda, nullptr,
+                                      reinterpret_cast<double*>(smem_raw));
     __syncthreads();
   }
   // ---- the three directions' sum, -1, the Jacobian, output / LSERK-W2 stage
@@ -369,24 +312,23 @@ k_volume_wfx(const double* __restrict__ U, const double* __restrict__ Pvol, cons
       rk.U[g] = rk.U[g] + utmp * rk.b_dt;
     }
   };
+  if (!sc.ok) {
+    for (int t = tid; t < 5 * n3; t += NT) put(t, __longlong_as_double(A[t]));
+    return;
+  }
 #pragma unroll 1
   for (int node = tid; node < n3; node += NT) {
     double ut[5];
-    if (sc.ok) {
-      const fx64* const a = A + vsw<NP>(node);
-      const double c = -Me[9 * n3 + node];
-      const int ch = __double2hiint(c), cl = __double2loint(c);
+    const fx64* const a = A + vsw<NP>(node);
+    const double c = -Me[9 * n3 + node];
+    const int ch = __double2hiint(c), cl = __double2loint(c);
 #pragma unroll
-      for (int v = 0; v < 5; ++v) {
-        fx64 r = 0;
+    for (int v = 0; v < 5; ++v) {
+      fx64 r = 0;
 #pragma unroll
-        for (int d = 0; d < 3; ++d) r += fx_sar(a[(5 * d + v) * n3], min(sc.d[d].t[v] - sc.t[v], 63));
-        const int k = sc.t[v] + wb.sD - 64 + wb.S;
-        ut[v] = __ll2double_rn(r) * __hiloint2double(ch - (k << 20), cl);
-      }
-    } else {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) ut[v] = __longlong_as_double(A[v * n3 + vsw<NP>(node)]);
+      for (int d = 0; d < 3; ++d) r += fx_sar(a[(5 * d + v) * n3], min(sc.d[d].t[v] - sc.t[v], 63));
+      const int k = sc.t[v] + wb.sD - 64 + wb.S;
+      ut[v] = __ll2double_rn(r) * __hiloint2double(ch - (k << 20), cl);
     }
     if constexpr (NP <= 5) {
       // into the node's own slots

@@ -101,3 +101,52 @@ def test_viscous_rows_of_the_weak_form(N, form):
     g, o = both(gx.config(N=N, R=R, parabolic=True, mu0=1e3, **FORMS[form]), m, U)
     r = rows(g, o)
     assert max(r[1:4]) <= 3e-14 and max(r[0], r[4]) <= 1e-13, r
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf])
+@pytest.mark.parametrize("parab", [False, True], ids=["euler", "ns"])
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("N", [2, 5])
+def test_non_finite_values_spread_as_in_fp64(N, form, parab, bad):
+    """The nodes that a value without a number reaches (its lines, the lifting's lines, the neighbours' faces) are the
+    oracle's, and the others keep their values."""
+    kw = dict(FORMS[form], Riemann="roe")
+    m = mesh(N, kw, (4, 2, 2))
+    U = noisy(m, "nonfinite", (2 * math.pi,) * 3)
+    U[5, 1, 1, 1, 4] = bad
+    cfg = gx.config(N=N, R=R, **(dict(kw, parabolic=True, mu0=1e-3) if parab else kw))
+    g, o = both(cfg, m, U)
+    fine = np.isfinite(o).all(-1)
+    assert fine.any() and not fine.all()
+    assert np.array_equal(np.isfinite(g).all(-1), fine)
+    assert max(rows(g[fine], o[fine])) <= 1e-12, rows(g[fine], o[fine])
+
+
+@pytest.mark.parametrize("form", ["pi", "kg", "weak", "gauss"])
+@pytest.mark.parametrize("N", [3, 7])
+def test_refused_elements_cost(N, form):
+    """A mesh of elements outside the scales takes what the FP64 kernel takes: up to 3.4 times the fixed-point volume
+    kernel in the kernels' own times, 6 with a margin for clocks."""
+    import ctypes
+    from galaexi_gb300 import _native as nat
+
+    kw = FORMS[form]
+    m = mesh(N, kw, (12, 12, 12) if N == 7 else (24, 24, 24))
+    U = gx.tgv_state(m, mach=0.1, R=R)
+    x = m.Elem_xGP[..., 0]
+    lo, hi = x.min(axis=(1, 2, 3), keepdims=True), x.max(axis=(1, 2, 3), keepdims=True)
+    states = {"ordinary": U, "refused": U * (2000.0 ** ((x - lo) / (hi - lo)))[..., None]}
+    t = {}
+    for name, s in states.items():
+        op = gx.DG(gx.config(N=N, R=R, parabolic=True, mu0=1e-3, **kw), m)
+        u = torch.from_numpy(np.ascontiguousarray(s)).cuda()
+        k = torch.zeros_like(u)
+        out = (ctypes.c_double * 5)()
+        best = math.inf
+        for _ in range(4):
+            nat.check(nat.lib().dg_profile_stage(op._h, ctypes.c_void_p(u.data_ptr()), ctypes.c_void_p(k.data_ptr()), 0.0, 4,
+                                                 out, op._stream()), "profile")
+            best = min(best, out[3])
+        op.close()
+        t[name] = best
+    assert t["refused"] <= 6.0 * t["ordinary"], t
