@@ -117,6 +117,11 @@ __device__ __forceinline__ double fx_to_double(fx64 t, fx64 m) {
   return __hiloint2double((dh & 0x7ff00000) ? dh - (s << 20) : 0, __double2loint(d));
 }
 
+// log2 of the ratio of the largest and smallest |M_d| of an element, from MetL
+__device__ __forceinline__ float fx_flatness(const float* MetL) {
+  return fmaxf(MetL[0], fmaxf(MetL[1], MetL[2])) - fminf(MetL[0], fminf(MetL[1], MetL[2]));
+}
+
 // warp maximum / minimum of a magnitude word, combined over the block in shared memory (initialised by
 // the caller; a block barrier follows)
 __device__ __forceinline__ void fx_block_max(unsigned v, unsigned* s) {

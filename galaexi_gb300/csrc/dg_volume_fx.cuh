@@ -86,6 +86,13 @@ __device__ __forceinline__ float fx_lse(float a, float b) {
 // 2^63.  Smaller contributions are shifted right to the scale that the largest allows.  The momentum rows c of a
 // direction differ in their pressure term p M_d,c (flat elements: a direction's large metric terms meet p in one
 // row only), so each row has its own last shift.
+// What a row loses is the distance from its own terms to the element's largest, so elements where that can be more
+// than the eight bits that the range has over FP64 take the FP64 sums: densities or pressures that differ by 2^8,
+// elements flatter than about 19:1 (their |M_d||u| stands against M_d.u of the flat direction; errors of the worst
+// row at 16:1, 64:1 and 256:1 at N = 2: 0.9, 2.4 and 10 times the FP64 kernel's), viscous stresses above four times
+// the pressure (there a momentum row with a small velocity has nothing of the size of the largest one's terms:
+// up to 2 times).  rho |u|^2 above the pressure costs nothing: the pressure itself, a difference of energies, has
+// the round-off of the larger.
 template <int SPLIT, int PARAB>
 __device__ __forceinline__ void vol_fx_scales(const unsigned* mag, const float* MetL, VolFxScale& S, int lane) {
   const int d = min(lane, 2);
@@ -98,6 +105,7 @@ __device__ __forceinline__ void vol_fx_scales(const unsigned* mag, const float* 
   const float Lr = fx_log2(mag[X_RHO]), La = fx_log2(mag[X_AUX]), Lp = fx_log2(mag[X_P]);
   const float Lu = 0.5f * __log2f(__uint_as_float(mag[X_U2])) + 1e-4f, LM = ok ? MetL[d] : 0.f;
   const float Lt = fx_log2(mag[X_TAU]) + 0.8f, Lq = fx_log2(mag[X_TQ]) + 0.8f;
+  ok = ok && fx_flatness(MetL) <= 4.25f && (!PARAB || Lt <= Lp + 2.8f);
   const int ev = (int)floorf(Lu) + 1, eM = (int)floorf(LM) + 1;
   const int s_rho = 61 - fx_exp(mag[X_RHO]), s_vel = 59 - ev, sM = 59 - eM;
   const int s_tau = 59 - fx_exp(mag[X_TAU]), s_tq = 59 - fx_exp(mag[X_TQ]);

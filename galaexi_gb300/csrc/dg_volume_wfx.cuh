@@ -57,7 +57,9 @@ enum { W_M2, W_U2, W_P, W_E, W_TAU, W_TQ, W_F, W_V = W_F + 15, W_R, W_NMAX, W_PM
 // row are shifted to it at the end; Mm is shifted to the scale of M p before its product with v.
 // Elements whose densities differ by more than 2^3 to 2^4 take the FP64 sums: at one pressure and velocity, rho u and
 // (E+p)/rho have their maxima at opposite nodes, and the energy row's bound is above its products by the contrast
-// (errors of the worst row, contrasts 8, 16, 64, 256: 0.65, 1.2, 2.4 and 5 times the FP64 kernel's).
+// (errors of the worst row, contrasts 8, 16, 64, 256: 0.65, 1.2, 2.4 and 5 times the FP64 kernel's).  So do flat
+// elements, from 10:1 on here (8:1, 16:1, 64:1 and 256:1 at N = 2: 0.9, 1.1, 3.9 and 13 times), and those whose stresses exceed
+// the pressure as there (vol_fx_scales; 4 to 6 times).
 template <int PARAB>
 __device__ __forceinline__ void vol_wfx_scales(const unsigned* mag, const float* MetL, VolWfxScale& S, int lane) {
   const int d = min(lane, 2);
@@ -73,6 +75,7 @@ __device__ __forceinline__ void vol_wfx_scales(const unsigned* mag, const float*
   const float Lp = fx_log2(mag[W_P]), LE = fx_log2(mag[W_E]);
   const float Lt = fx_log2(mag[W_TAU]) + 0.8f, Lq = fx_log2(mag[W_TQ]) + 0.8f;
   const float LV = LM + Lm;
+  ok = ok && fx_flatness(MetL) <= 3.25f && (!PARAB || Lt <= Lp + 2.8f);
   VolWfxDir o;
   o.sM = 59 - ((int)floorf(LM) + 1);
   const int s_m = 59 - ((int)floorf(Lm) + 1), s_v = 59 - ((int)floorf(Lu) + 1);
