@@ -634,7 +634,7 @@ int dg_set_mesh(dg_ctx* ctx, int nElems, int nSides, int nBCSides, const double*
     const dg_config& c = ctx->cfg;
     const bool gl = c.node_type == DG_NODETYPE_GAUSS_LOBATTO;
     gxc::DBuf<int> flags;
-    if (!ctx->MetL.alloc((size_t)nElems * 16) || !flags.alloc(1)) { set_error("cudaMalloc mesh"); return DG_ERR_ALLOC; }
+    if (!ctx->MetL.alloc((size_t)nElems * gx::kMetL) || !flags.alloc(1)) { set_error("cudaMalloc mesh"); return DG_ERR_ALLOC; }
     int f = 0;
     cudaError_t err = cudaMemset(flags.p, 0, sizeof(int));
     if (err == cudaSuccess) err = gxc::mesh_scales(ctx->d.Met.p, ctx->d.Fgeo.p, ctx->E2S.p, nElems, n, gl, ctx->MetL.p, flags.p);

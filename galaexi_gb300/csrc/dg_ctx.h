@@ -122,8 +122,8 @@ struct dg_ctx {
   int sms = 0;             // SMs of the device
   int lines_grid = 0;      // blocks of the persistent line volume kernel (SMs x resident blocks), on first use
   int prolong_grid = 0;    // blocks of the persistent prolongation kernel of the mixed form, on first use
-  // FP64 form, block fixed-point kernels: log2 of the largest |M_d| (3), |M_d,c| (9), SurfElem and
-  // |sJ| of each element (16 words; kFxNoScale: outside the range of the scales), and the basis as limbs (VolFxBasis)
+  // FP64 form, block fixed-point kernels: log2 of the largest metric terms of each element (kMetL words,
+  // dg_volume_fx.cuh), and the basis as limbs (VolFxBasis)
   gxc::DBuf<float> MetL;
   bool lift_fx = false;    // fixed-point lifting: strong non-conservative form, no element flatter than 2^8
   bool face_exact = false; // SurfElem n = +-M of both elements' face nodes to the last bits (affine elements)

@@ -18,20 +18,21 @@ __device__ void block_max(double x, unsigned long long* s) {
 __device__ double larger(double a, double b) { return b <= a ? a : b; }  // keeps a NaN that comes second
 __device__ double keep(double a, double b) { return a == a ? larger(a, b) : a; }
 
-// MetL[e][16] (dg_ctx.h); flags: bit 0 an element flatter than 2^8, bit 1 SurfElem n differs from the metric terms
+// MetL[e][kMetL] (dg_volume_fx.cuh); flags: bit 0 an element flatter than 2^8, bit 1 SurfElem n differs from the metric terms
 // of an element's face nodes (Gauss-Lobatto nodes; +- by side and flip) by more than 4.5e-16 SurfElem somewhere.
 // Memory bound: one block per element reads the geometry once.
 __global__ void __launch_bounds__(128)
 k_mesh_scales(const double* __restrict__ Met, const double* __restrict__ Fgeo, const int* __restrict__ E2S, int n, int gl,
               float* __restrict__ MetL, int* __restrict__ flags) {
   const int n2 = n * n, n3 = n2 * n, N = n - 1;
-  __shared__ unsigned long long big[16];  // 0-2 |M_d|^2, 3-11 M_d,c^2, 12 SurfElem, 13 |sJ|, 14 1/|sJ|, 15 |n_c|
-  if (threadIdx.x < 16) big[threadIdx.x] = 0ull;
+  constexpr int NW = 19;
+  __shared__ unsigned long long big[NW];  // 0-2 |M_d|^2, 3-11 M_d,c^2, 12 SurfElem, 13 |sJ|, 14 1/|sJ|, 15 |n_c|, 16-18 |SurfElem n_c|
+  if (threadIdx.x < NW) big[threadIdx.x] = 0ull;
   __syncthreads();
   const size_t e = blockIdx.x;
   const double* const m = Met + e * 10 * n3;
-  double w[16];
-  for (int c = 0; c < 16; ++c) w[c] = 0.;
+  double w[NW];
+  for (int c = 0; c < NW; ++c) w[c] = 0.;
   for (int t = threadIdx.x; t < n3; t += blockDim.x) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -65,23 +66,27 @@ k_mesh_scales(const double* __restrict__ Met, const double* __restrict__ Fgeo, c
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       w[15] = keep(w[15], fabs(f[c * n2]));
+      w[16 + c] = keep(w[16 + c], fabs(se * f[c * n2]));
       differs = differs || !(fabs(__dsub_rn(sg * se * f[c * n2], m[(size_t)(3 * dir + c) * n3 + node])) <= se * 4.5e-16);
     }
   }
 #pragma unroll
-  for (int c = 0; c < 16; ++c) block_max(w[c], &big[c]);
+  for (int c = 0; c < NW; ++c) block_max(w[c], &big[c]);
   if (__syncthreads_or(gl && differs) && threadIdx.x == 0) atomicOr(flags, 2);
   if (threadIdx.x != 0) return;
   auto at = [&](int c) { return __longlong_as_double((long long)big[c]); };
   bool fine = at(13) < 1e45 && at(14) < 1e45;
   for (int d = 0; d < 3; ++d) fine = fine && at(d) > 1e-90 && at(d) < 1e90;
-  float* const l = MetL + e * 16;
+  float* const l = MetL + e * gx::kMetL;
   for (int c = 0; c < 12; ++c)
     l[c] = !fine ? gx::kFxNoScale : (at(c) > 1e-90 ? (float)(0.5 * log2(at(c)) + 1e-5) : -150.f);
   const bool face = fine && at(12) > 1e-45 && at(12) < 1e45 && at(15) <= 1. + 1e-9;
   l[12] = face ? (float)(log2(at(12)) + 1e-5) : gx::kFxNoScale;
   l[13] = face ? (float)(log2(at(13)) + 1e-5) : gx::kFxNoScale;
-  l[14] = l[15] = 0.f;
+  for (int c = 0; c < 3; ++c) {
+    const float f = face && at(16 + c) > 1e-45 ? (float)(log2(at(16 + c)) + 1e-5) : -150.f;
+    l[14 + c] = fmaxf(fmaxf(l[3 + c], f), fmaxf(l[6 + c], l[9 + c]));
+  }
   if (fmaxf(l[0], fmaxf(l[1], l[2])) - fminf(l[0], fminf(l[1], l[2])) > 8.f) atomicOr(flags, 1);
 }
 

@@ -6,7 +6,7 @@
 // reads the density gradient).  On Gauss-Lobatto nodes the surface term of a node on a face is
 //   L_hat 0.5 SurfElem n (P_slave - P_master),   SurfElem n = +- M_dir of the element's own face node
 // up to the round-off of the mesh's metric terms.  Where the two are equal to the last bits (EXACT, checked on
-// the host for the mesh: affine elements), the term is added to the reference derivative of the face's
+// the device for the mesh, k_mesh_scales: affine elements), the term is added to the reference derivative of the face's
 // direction before the metric terms: y_dir += N(N+1)/4 (neighbour - own) on the plus face, (own - neighbour)
 // on the minus face, L_hat = N(N+1)/2; otherwise it is added in FP64 by face-node threads with the face's own
 // geometry.  The gradients are g_d = sJ sum_dir M_dir,d y_dir.
@@ -20,6 +20,7 @@
 #include "dg_fx.cuh"
 #include "dg_kernels.cuh"
 #include "dg_lines.cuh"
+#include "dg_volume_fx.cuh"
 
 namespace gx {
 
@@ -153,7 +154,8 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
     for (int v = 0; v < 4; ++v) fx_block_max(m[v], &mag[v]);
   }
   __syncthreads();
-  bool ok = MetL[(size_t)e * 16] < 200.f;
+  const float* const ml = MetL + (size_t)e * kMetL;
+  bool ok = ml[0] < 200.f;
 #pragma unroll
   for (int v = 0; v < 4; ++v) ok = ok && mag[v] < ((1022u + 150u) << 20);
   if (ok) {
@@ -232,8 +234,11 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
     __syncthreads();
   }
   // ---- node by node: sJ M digits (< 2^58), the gradients with 2 bits below the digits' unit, and their traces
-  const float Lmax = fmaxf(MetL[(size_t)e * 16], fmaxf(MetL[(size_t)e * 16 + 1], MetL[(size_t)e * 16 + 2]));
-  const int sM = 59 - ((int)floorf(Lmax) + 1), r_M = fx_r0(sM);
+  // (one scale for each component of the gradient: in a flat element that of the flat direction meets the large
+  // metric terms, the others the small ones)
+  int sM[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) sM[d] = ok ? 59 - ((int)floorf(ml[14 + d]) + 1) : 0;
 #pragma unroll 1
   for (int it = 0; it < NPT; ++it) {
     const int node = tid + it * NT;
@@ -247,7 +252,7 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
 #pragma unroll
       for (int c = 0; c < 9; ++c) {
         FxDot p;
-        p.add(fd_from(Me[c * n3 + node], r_M), J);
+        p.add(fd_from(Me[c * n3 + node], fx_r0(sM[c % 3])), J);
         M[c] = fd_split(p.sum());
       }
       const int sn = vsw<NP>(node);
@@ -256,14 +261,14 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
         FxDig y[3];
 #pragma unroll
         for (int dir = 0; dir < 3; ++dir) y[dir] = fd_split(Y[(dir * 4 + v) * n3 + sn]);
-        // g = r 2^k: scales of sJ M, of y, of the product
-        const int k = -((sM + 59 - ej - 60) + (57 - fx_exp(mag[v]) + lb.sD - 60 + 3) - 60 + 2);
+        // g = r 2^(k - sM): scales of sJ M, of y, of the product
+        const int k = -((59 - ej - 60) + (57 - fx_exp(mag[v]) + lb.sD - 60 + 3) - 60 + 2);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           FxDot p;
 #pragma unroll
           for (int dir = 0; dir < 3; ++dir) p.add(y[dir], M[3 * dir + d]);
-          g[d * 4 + v] = fx_scaled(p.sum<2>(), k);
+          g[d * 4 + v] = fx_scaled(p.sum<2>(), k - sM[d]);
         }
       }
     } else {

@@ -114,7 +114,7 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
   __syncthreads();
   const double* const Pe = Pvol + (size_t)e * 7 * n3;
   const double* const Me = Met + (size_t)e * 10 * n3;
-  const float* const ml = MetL + (size_t)e * 16;
+  const float* const ml = MetL + (size_t)e * kMetL;
   auto liftc = [](int v) { return v == 3 ? 5 : v + 1; };
   auto side_of = [](int dir, int pm) {
     return dir == 0 ? (pm == 0 ? L_XI_MINUS : L_XI_PLUS)
@@ -123,8 +123,9 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
   // node l of line (a, b) of a direction
   auto line = [](int dir, int ab) { return dir == 0 ? n * ab : (dir == 1 ? (ab % n) + n2 * (ab / n) : ab); };
   bool ok = ml[0] < 200.f && ml[12] < 200.f;
-  const float Lmax = fmaxf(ml[0], fmaxf(ml[1], ml[2]));
-  const int sM = ok ? 58 - ((int)floorf(Lmax) + 1) : 0, sE = ok ? 58 - ((int)floorf(ml[12]) + 1) : 0;
+  int sM[3];  // of M_dir,d and SurfElem n_d, for each component d of the gradient
+#pragma unroll
+  for (int d = 0; d < 3; ++d) sM[d] = ok ? 58 - ((int)floorf(ml[14 + d]) + 1) : 0;
   const int sJ = ok ? 59 - ((int)floorf(ml[13]) + 1) : 0;
   // ---- one scale per variable: the largest magnitude of the element and of both traces on its faces
   {
@@ -153,7 +154,8 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
   __syncthreads();
 #pragma unroll
   for (int v = 0; v < 4; ++v) ok = ok && mag[v] < ((1022u + 150u) << 20);
-  // Scales (powers of two): |x| < 2^57, |M| < 2^58, SurfElem n < 2^58, |sJ| < 2^59; y = D x below 2^60 (as in
+  // Scales (powers of two): |x| < 2^57, |M| < 2^58 and SurfElem n < 2^58 for each component of the gradient (in flat
+  // elements they differ by the aspect ratio), |sJ| < 2^59; y = D x below 2^60 (as in
   // k_lift_fx), F = (SurfElem/2 n) dx below 2^59.  From here on the scale follows the largest |y| and |F| of the
   // element, which are smaller than their bounds by the smoothness of the field (with the bounds alone 4 to 16
   // times the FP64 kernel's error on smooth viscous flow): y and F are shifted to one scale of the sums M y (three
@@ -185,12 +187,16 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
       FxDig dx[4], G[3];
 #pragma unroll
       for (int v = 0; v < 4; ++v) dx[v] = fd_from(pr[liftc(v) * n2], r0[v]) - fd_from(pl[liftc(v) * n2], r0[v]);
-      const FxDig se = fd_from(fg[9 * n2], fx_r0(sE));
+      const int es9 = fx_exp(fx_mag(fg[9 * n2]));
+      const FxDig se = fd_from(fg[9 * n2], fx_r0(58 - es9));
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
+        // SurfElem and n_d with all their bits, then to the component's scale
+        const double nd = fg[d * n2];
+        const int en = fx_exp(fx_mag(nd));
         FxDot s;
-        s.add(fd_from(fg[d * n2], fx_r0(58)), se);
-        G[d] = fd_split(s.sum<2>());
+        s.add(fd_from(nd, fx_r0(58 - en)), se);
+        G[d] = fd_scaled(s.sum<2>(), max(sM[d] - (58 - es9 - en), -63));
       }
       fx64* const Fo = F + f * 12 * n2 + ab;
 #pragma unroll
@@ -275,7 +281,8 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
     __syncthreads();
     {
       const int v = tid & 3, ev = fx_exp(mag[v]), bY = fx_bits(magY[v]), bF = fx_bits(magF[v]);
-      const int s_v = gb.d.sD - ev + sM - 60, s_F = sE + 1 - ev, s_s = s_F + gb.sL - 60;  // of M y / 2^60, Lhat F / 2^60
+      // (without the components' sM)
+      const int s_v = gb.d.sD - ev - 60, s_F = 1 - ev, s_s = s_F + gb.sL - 60;  // of M y / 2^60, Lhat F / 2^60
       const int s_g = min(s_v + min(60 - bY, 30), s_s + min(59 - bF, 30)), s_G = s_g + sJ - 60;
       LiftGfxScale o;
       o.KY = max(s_g - s_v, -63);
@@ -306,7 +313,7 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
       const int ix[3] = {i, j, k}, ab[3] = {j + n * k, i + n * k, i + n * j};
       FxDig M[9];
 #pragma unroll
-      for (int c = 0; c < 9; ++c) M[c] = fd_from(Me[c * n3 + node], fx_r0(sM));
+      for (int c = 0; c < 9; ++c) M[c] = fd_from(Me[c * n3 + node], fx_r0(sM[c % 3]));
       const FxDig jc = fd_unpack(J[node]);
       FxDig lm[3], lp[3];
       if constexpr (GAUSS) {
@@ -340,7 +347,7 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
           FxDotU g;
           g.add(fd_split(p.sum()), jc);
           const fx64 gt = g.sum();
-          G[(d * 5 + 1 + v) * n3] = fx_scaled(gt, o.kG);
+          G[(d * 5 + 1 + v) * n3] = fx_scaled(gt, o.kG - sM[d]);
           // for the traces: BR2 prolongs the volume part only
           if constexpr (BR2) {
             FxDotU h;
@@ -416,7 +423,7 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
             s.add(fd_unpack(F[((dir * 2 + pm) * 12 + d * 4 + v) * n2 + li]), fd_unpack(Cb[(dir * 2 + pm) * n2 + li]));
             t = fx_sar(t, o.kt) + fx_sar(s.sum(), o.kb);
           }
-          out[pm][d * 5 * n2] = fx_scaled(t, -o.s_o);
+          out[pm][d * 5 * n2] = fx_scaled(t, -o.s_o - sM[d]);
         }
       }
     } else {

@@ -54,9 +54,10 @@ template <int NP, typename R, int SPLIT, typename S> struct UseVolFx {
 template <int NP> struct VolFxBasis {
   FxLimb Q[NP * NP], iw[NP];
 };
-// MetL[e][16]: log2 of the largest |M_d| (2-norm; 3) of the element, of its largest |M_d,c| (9), SurfElem and |sJ|
-// (one each), or kFxNoScale where its geometry is outside the range the scales are made for (2^-150 .. 2^150); such
+// MetL[e][kMetL]: log2 of the largest |M_d| (2-norm; 3) of the element, of its largest |M_d,c| (9), SurfElem and |sJ|
+// (one each), of the largest |M_d,c| and |SurfElem n_c| over directions and faces (3), or kFxNoScale where its geometry is outside the range the scales are made for (2^-150 .. 2^150); such
 // elements take the FP64 path
+constexpr int kMetL = 17;
 constexpr float kFxNoScale = 1e9f;
 
 // shifts of one direction (see vol_fx_scales) and the scales of its five rows
@@ -488,7 +489,7 @@ k_volume_fx(const double* __restrict__ U, const double* __restrict__ Pvol, const
     fx_block_min(pmin, &mag[X_PMIN]);
   }
   __syncthreads();
-  if (warp == 0) vol_fx_scales<SPLIT, PARAB>(mag, MetL + (size_t)e * 16, sc, lane);
+  if (warp == 0) vol_fx_scales<SPLIT, PARAB>(mag, MetL + (size_t)e * kMetL, sc, lane);
   __syncthreads();
   double* const Us = reinterpret_cast<double*>(smem_raw);  // Ut of the element, [node][5], at the end
   if (sc.ok) {

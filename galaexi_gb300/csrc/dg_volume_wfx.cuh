@@ -200,7 +200,7 @@ k_volume_wfx(const double* __restrict__ U, const double* __restrict__ Pvol, cons
     fx_block_min(rmin, &mag[W_RMIN]);
   }
   __syncthreads();
-  if (tid < 32) vol_wfx_scales<PARAB>(mag, MetL + (size_t)e * 16, sc, tid);
+  if (tid < 32) vol_wfx_scales<PARAB>(mag, MetL + (size_t)e * kMetL, sc, tid);
   __syncthreads();
   if (sc.ok) {
     // ---- contravariant fluxes
