@@ -40,40 +40,61 @@ template <int NP> struct LiftFxBasis {
   int sD;
 };
 
-// the FP64 lifting of one node, from global memory: for elements whose values do not fit one scale
-template <int NP>
-__device__ __noinline__ void lift_node_fp64(const double* Pe, const double* Me, const double* Pf, const double* Fgeo,
-                                            const int* es, int nSides, const double* D, double Lhat, int node,
-                                            double g[12]) {
-  constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP, N = NP - 1;
-  const int liftc[4] = {1, 2, 3, 5};
-  const int ijk[3] = {node % n, (node / n) % n, node / n2};
-  const double sj = Me[(size_t)9 * n3 + node];
-  for (int c = 0; c < 12; ++c) g[c] = 0.;
+// u, v, w, T in FP64 to X [4][n3], and the derivatives of the lines of all directions to Y [3][4][n3] (elements whose
+// values do not fit one scale): the FP64 kernel's sums, by the block
+template <int NP, int NT>
+__device__ __noinline__ void lift_lines_fp64(const double* Pe, const double* D, double* X, double* Y) {
+  constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP;
+  __syncthreads();
 #pragma unroll 1
-  for (int dir = 0; dir < 3; ++dir) {
-    const int step = dir == 0 ? 1 : (dir == 1 ? n : n2), i = ijk[dir], base = node - i * step;
-    double y[4] = {0., 0., 0., 0.};
-#pragma unroll 1
-    for (int l = 0; l < n; ++l)
-      for (int v = 0; v < 4; ++v) y[v] = y[v] + D[i + n * l] * Pe[liftc[v] * n3 + base + l * step];
-    for (int d = 0; d < 3; ++d)
-      for (int v = 0; v < 4; ++v) g[d * 4 + v] = g[d * 4 + v] + sj * Me[(size_t)(3 * dir + d) * n3 + node] * y[v];
+  for (int t = threadIdx.x; t < 4 * n3; t += NT) {
+    const int v = t / n3, node = t - v * n3;
+    X[v * n3 + vsw<NP>(node)] = Pe[(v == 3 ? 5 : v + 1) * n3 + node];
   }
+  __syncthreads();
 #pragma unroll 1
-  for (int f = 0; f < 6; ++f) {
-    int ls, a, b;
-    if (!node_face<NP>(f, ijk[0], ijk[1], ijk[2], ls, a, b)) continue;
-    const int side = es[2 * (ls - 1)], flip = es[2 * (ls - 1) + 1];
-    int p, q;
-    s2v2_inv(N, a, b, flip, ls, p, q);
-    const double* pm = Pf + (size_t)side * 6 * n2 + p + n * q;
-    const double* ps = pm + (size_t)nSides * 6 * n2;
-    const double* fg = Fgeo + (size_t)side * 10 * n2 + p + n * q;
-    const double w = Lhat * 0.5 * fg[9 * n2] * sj;
-    for (int d = 0; d < 3; ++d)
-      for (int v = 0; v < 4; ++v)
-        g[d * 4 + v] = g[d * 4 + v] + (ps[liftc[v] * n2] - pm[liftc[v] * n2]) * (w * fg[d * n2]);
+  for (int t = threadIdx.x; t < 12 * n2; t += NT) {
+    const int dv = t / n2, li = t - dv * n2, dir = dv >> 2, step = dir == 0 ? 1 : (dir == 1 ? n : n2);
+    const int base = dir == 0 ? n * li : (dir == 1 ? (li % n) + n2 * (li / n) : li);
+    const double* const Xv = X + (dv & 3) * n3;
+    double x[n];
+#pragma unroll
+    for (int l = 0; l < n; ++l) x[l] = Xv[vsw<NP>(base + l * step)];
+#pragma unroll 2
+    for (int i = 0; i < n; ++i) {
+      double y = 0.;
+#pragma unroll
+      for (int l = 0; l < n; ++l) y = y + D[i + n * l] * x[l];
+      Y[dv * n3 + vsw<NP>(base + i * step)] = y;
+    }
+  }
+  __syncthreads();
+}
+// a node's gradients (volume part) from its derivatives, g[d * 4 + v]; then those of all nodes in the derivatives' place
+template <int NP>
+__device__ __forceinline__ void lift_node_fp64(const double* Me, const double* Y, int node, double g[12]) {
+  constexpr int n3 = NP * NP * NP;
+  const double sj = Me[(size_t)9 * n3 + node];
+#pragma unroll
+  for (int c = 0; c < 12; ++c) g[c] = 0.;
+#pragma unroll
+  for (int dir = 0; dir < 3; ++dir)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double m = sj * Me[(size_t)(3 * dir + d) * n3 + node];
+#pragma unroll
+      for (int v = 0; v < 4; ++v) g[d * 4 + v] = g[d * 4 + v] + m * Y[(dir * 4 + v) * n3 + vsw<NP>(node)];
+    }
+}
+template <int NP, int NT>
+__device__ __noinline__ void lift_nodes_fp64(const double* Me, double* Y) {
+  constexpr int n3 = NP * NP * NP;
+#pragma unroll 1
+  for (int node = threadIdx.x; node < n3; node += NT) {
+    double g[12];
+    lift_node_fp64<NP>(Me, Y, node, g);
+#pragma unroll
+    for (int c = 0; c < 12; ++c) Y[c * n3 + vsw<NP>(node)] = g[c];
   }
 }
 
@@ -232,6 +253,10 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
       }
     }
     __syncthreads();
+  } else {
+    double* const Yd = reinterpret_cast<double*>(Y);
+    lift_lines_fp64<NP, NT>(Pe, D, Yd + 12 * n3, Yd);
+    lift_nodes_fp64<NP, NT>(Me, Yd);
   }
   // ---- node by node: sJ M digits (< 2^58), the gradients with 2 bits below the digits' unit, and their traces
   // (one scale for each component of the gradient: in a flat element that of the flat direction meets the large
@@ -240,41 +265,37 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
 #pragma unroll
   for (int d = 0; d < 3; ++d) sM[d] = ok ? 59 - ((int)floorf(ml[14 + d]) + 1) : 0;
 #pragma unroll 1
-  for (int it = 0; it < NPT; ++it) {
+  for (int it = 0; it < (ok ? NPT : 0); ++it) {
     const int node = tid + it * NT;
     if (node >= n3) break;
     double g[12];
-    if (ok) {
-      const double sj = Me[9 * n3 + node];
-      const int ej = fx_exp(fx_mag(sj));
-      const FxDig J = fd_from(sj, fx_r0(59 - ej));  // sj 2^(59-ej) in [2^58, 2^59)
-      FxDig M[9];
+    const double sj = Me[9 * n3 + node];
+    const int ej = fx_exp(fx_mag(sj));
+    const FxDig J = fd_from(sj, fx_r0(59 - ej));  // sj 2^(59-ej) in [2^58, 2^59)
+    FxDig M[9];
 #pragma unroll
-      for (int c = 0; c < 9; ++c) {
-        FxDot p;
-        p.add(fd_from(Me[c * n3 + node], fx_r0(sM[c % 3])), J);
-        M[c] = fd_split(p.sum());
-      }
-      const int sn = vsw<NP>(node);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        FxDig y[3];
-#pragma unroll
-        for (int dir = 0; dir < 3; ++dir) y[dir] = fd_split(Y[(dir * 4 + v) * n3 + sn]);
-        // g = r 2^(k - sM): scales of sJ M, of y, of the product
-        const int k = -((59 - ej - 60) + (57 - fx_exp(mag[v]) + lb.sD - 60 + 3) - 60 + 2);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          FxDot p;
-#pragma unroll
-          for (int dir = 0; dir < 3; ++dir) p.add(y[dir], M[3 * dir + d]);
-          g[d * 4 + v] = fx_scaled(p.sum<2>(), k - sM[d]);
-        }
-      }
-    } else {
-      lift_node_fp64<NP>(Pe, Me, Pf, Fgeo, es, nSides, D, Lhat, node, g);
+    for (int c = 0; c < 9; ++c) {
+      FxDot p;
+      p.add(fd_from(Me[c * n3 + node], fx_r0(sM[c % 3])), J);
+      M[c] = fd_split(p.sum());
     }
-    if (EXACT || !ok) {
+    const int sn = vsw<NP>(node);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      FxDig y[3];
+#pragma unroll
+      for (int dir = 0; dir < 3; ++dir) y[dir] = fd_split(Y[(dir * 4 + v) * n3 + sn]);
+      // g = r 2^(k - sM): scales of sJ M, of y, of the product
+      const int k = -((59 - ej - 60) + (57 - fx_exp(mag[v]) + lb.sD - 60 + 3) - 60 + 2);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        FxDot p;
+#pragma unroll
+        for (int dir = 0; dir < 3; ++dir) p.add(y[dir], M[3 * dir + d]);
+        g[d * 4 + v] = fx_scaled(p.sum<2>(), k - sM[d]);
+      }
+    }
+    if constexpr (EXACT) {
       put_gradients<NP>(g, node, (size_t)e, es, nSides, Gvol, Gf);
     } else {
       // this node's derivatives are read: its gradients take their place
@@ -282,7 +303,7 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
       for (int c = 0; c < 12; ++c) Y[c * n3 + vsw<NP>(node)] = __double_as_longlong(g[c]);
     }
   }
-  if (!EXACT && ok) {
+  if (!EXACT || !ok) {
     __syncthreads();
     // surface part, one thread per face node, one normal direction per pass (its two faces share no node)
 #pragma unroll 1

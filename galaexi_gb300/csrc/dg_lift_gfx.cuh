@@ -45,45 +45,57 @@ struct LiftGfxScale {
   int KY, KF, kG, s_o, kt, kb;
 };
 
-// The FP64 lifting of one node, from global memory (elements whose values do not fit one scale): gv the volume
-// part, gt with the surface part
-template <int NP, bool GAUSS>
-__device__ __noinline__ void lift_gen_node_fp64(const double* Pe, const double* Me, const double* Pf, const double* Fgeo,
-                                                const int* es, int nSides, const double* D, const double* Lhm,
-                                                const double* Lhp, int node, double gv[12], double gt[12]) {
+// The FP64 lifting by the block (elements whose values do not fit one scale): the gradients to Gvol, those that the
+// traces are formed from (BR2: the volume part) to Y.  X, F: shared memory as in the kernel below
+template <int NP, bool GAUSS, bool BR2, int NT>
+__device__ __noinline__ void lift_gen_fp64(const double* Pe, const double* Me, const double* Pf, const double* Fgeo,
+                                           const int* es, int nSides, const double* D, const double* Lhm,
+                                           const double* Lhp, double* Ge, double* X, double* F, double* Y) {
   constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP, N = NP - 1;
   const int liftc[4] = {1, 2, 3, 5};
-  const int ijk[3] = {node % n, (node / n) % n, node / n2};
-  const double sj = Me[(size_t)9 * n3 + node];
-  for (int c = 0; c < 12; ++c) gv[c] = 0.;
 #pragma unroll 1
-  for (int dir = 0; dir < 3; ++dir) {
-    const int step = dir == 0 ? 1 : (dir == 1 ? n : n2), i = ijk[dir], base = node - i * step;
-    double y[4] = {0., 0., 0., 0.};
-#pragma unroll 1
-    for (int l = 0; l < n; ++l)
-      for (int v = 0; v < 4; ++v) y[v] = y[v] + D[i + n * l] * Pe[liftc[v] * n3 + base + l * step];
-    for (int d = 0; d < 3; ++d)
-      for (int v = 0; v < 4; ++v) gv[d * 4 + v] = gv[d * 4 + v] + sj * Me[(size_t)(3 * dir + d) * n3 + node] * y[v];
-  }
-  for (int c = 0; c < 12; ++c) gt[c] = gv[c];
-#pragma unroll 1
-  for (int f = 0; f < 6; ++f) {
-    const int dir = f >> 1, pm = f & 1, l = ijk[dir];
-    if (!GAUSS && l != (pm == 0 ? 0 : N)) continue;
+  for (int t = threadIdx.x; t < 6 * n2; t += NT) {
+    const int f = t / n2, ab = t - f * n2, dir = f >> 1, pm = f & 1;
     const int ls = dir == 0 ? (pm == 0 ? L_XI_MINUS : L_XI_PLUS)
                             : (dir == 1 ? (pm == 0 ? L_ETA_MINUS : L_ETA_PLUS) : (pm == 0 ? L_ZETA_MINUS : L_ZETA_PLUS));
-    const int a = dir == 0 ? ijk[1] : ijk[0], b = dir == 2 ? ijk[1] : ijk[2];
     const int side = es[2 * (ls - 1)], flip = es[2 * (ls - 1) + 1];
     int p, q;
-    s2v2_inv(N, a, b, flip, ls, p, q);
-    const double* pl = Pf + (size_t)side * 6 * n2 + p + n * q;
-    const double* pr = pl + (size_t)nSides * 6 * n2;
-    const double* fg = Fgeo + (size_t)side * 10 * n2 + p + n * q;
-    const double w = (pm == 0 ? Lhm[l] : Lhp[l]) * 0.5 * fg[9 * n2] * sj;
-    for (int d = 0; d < 3; ++d)
-      for (int v = 0; v < 4; ++v)
-        gt[d * 4 + v] = gt[d * 4 + v] + (pr[liftc[v] * n2] - pl[liftc[v] * n2]) * (w * fg[d * n2]);
+    s2v2_inv(N, ab % n, ab / n, flip, ls, p, q);
+    const double* const pl = Pf + (size_t)side * 6 * n2 + p + n * q;
+    const double* const pr = pl + (size_t)nSides * 6 * n2;
+    const double* const fg = Fgeo + (size_t)side * 10 * n2 + p + n * q;
+    const double w = 0.5 * fg[9 * n2], nv[3] = {w * fg[0], w * fg[n2], w * fg[2 * n2]};
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const double fl = pr[liftc[v] * n2] - pl[liftc[v] * n2];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) F[(f * 12 + d * 4 + v) * n2 + ab] = fl * nv[d];
+    }
+  }
+  lift_lines_fp64<NP, NT>(Pe, D, X, Y);
+#pragma unroll 1
+  for (int node = threadIdx.x; node < n3; node += NT) {
+    double g[12];
+    lift_node_fp64<NP>(Me, Y, node, g);
+    if constexpr (BR2)
+#pragma unroll
+      for (int c = 0; c < 12; ++c) Y[c * n3 + vsw<NP>(node)] = g[c];
+    const double sj = Me[(size_t)9 * n3 + node];
+    const int ijk[3] = {node % n, (node / n) % n, node / n2};
+    const int ab[3] = {ijk[1] + n * ijk[2], ijk[0] + n * ijk[2], ijk[0] + n * ijk[1]};
+#pragma unroll
+    for (int f = 0; f < 6; ++f) {
+      const int dir = f >> 1, l = ijk[dir];
+      if (!GAUSS && l != ((f & 1) == 0 ? 0 : N)) continue;
+      const double w = sj * ((f & 1) == 0 ? Lhm[l] : Lhp[l]);
+#pragma unroll
+      for (int c = 0; c < 12; ++c) g[c] = g[c] + w * F[(f * 12 + c) * n2 + ab[dir]];
+    }
+#pragma unroll
+    for (int c = 0; c < 12; ++c) {
+      Ge[(c / 4 * 5 + 1 + c % 4) * n3 + node] = g[c];
+      if constexpr (!BR2) Y[c * n3 + vsw<NP>(node)] = g[c];
+    }
   }
 }
 
@@ -360,16 +372,9 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
       }
     }
   } else {
-#pragma unroll 1
-    for (int node = tid; node < n3; node += NT) {
-      double gv[12], gt[12];
-      lift_gen_node_fp64<NP, GAUSS>(Pe, Me, Pf, Fgeo, es, nSides, basis.D, basis.Lhm, basis.Lhp, node, gv, gt);
-#pragma unroll
-      for (int c = 0; c < 12; ++c) {
-        Gvol[(size_t)e * 15 * n3 + (c / 4 * 5 + 1 + c % 4) * n3 + node] = gt[c];
-        Y[c * n3 + vsw<NP>(node)] = __double_as_longlong(BR2 ? gv[c] : gt[c]);
-      }
-    }
+    lift_gen_fp64<NP, GAUSS, BR2, NT>(Pe, Me, Pf, Fgeo, es, nSides, basis.D, basis.Lhm, basis.Lhp,
+                                      Gvol + (size_t)e * 15 * n3, reinterpret_cast<double*>(X),
+                                      reinterpret_cast<double*>(F), reinterpret_cast<double*>(Y));
   }
   __syncthreads();
   // ---- traces on the two faces of a line

@@ -178,3 +178,27 @@ def test_stresses_above_the_pressure(form):
     g, o = both(gx.config(N=6, R=R, parabolic=True, mu0=1e3, **kw), m, U)
     r = rows(g, o)
     assert max(r[1:4]) <= 5e-14 and max(r[0], r[4]) <= 1e-13, r
+
+
+@pytest.mark.parametrize("which", ["all", "some"])
+@pytest.mark.parametrize("deform", [0.0, 0.05], ids=["affine", "curved"])
+@pytest.mark.parametrize("form", ["pi", "gauss", "gauss_br2", "pi_br2"])
+@pytest.mark.parametrize("N", [2, 5, 7])
+def test_lifting_outside_its_scales(N, form, deform, which):
+    """Temperatures above 2^150 (by the unit of the gas constant) in all elements or in some beside ordinary ones: the
+    lifting's FP64 sums.  The oracle's rows are within 5e-13 of 80 bits (noise of
+    1% on a flow of M = 0.1): bar four times that on affine elements.  On curved Gauss-Lobatto elements the FP64 kernels
+    themselves are up to 3.5e-12 from 80 bits in the momentum rows: the FP64 form's 1e-12 over all rows."""
+    kw = FORMS[form]
+    m = gx.Mesh(N, 1 if "NodeType" in kw else 2, 5, 2, 1, (-math.pi,) * 3, (math.pi,) * 3, deform=deform)
+    U = noisy(m, "lifting" + form, (2 * math.pi,) * 3)
+    gas = 1e-50
+    if which == "some":
+        gas = 71.4 / (0.4 * 2.0 ** 150)
+        U[2, ..., :4] *= 0.25  # four times the temperature
+    g, o = both(gx.config(N=N, R=gas, parabolic=True, mu0=0.1, **kw), m, U)
+    assert np.isfinite(o).all()
+    if deform:
+        assert np.linalg.norm(g - o) <= 1e-12 * np.linalg.norm(o)
+    else:
+        assert max(rows(g, o)) <= 2e-12, rows(g, o)
