@@ -40,6 +40,20 @@ template <int NP> struct LiftFxBasis {
   int sD;
 };
 
+// Elements that take the FP64 sums: those where a magnitude mag of u, v, w, T is outside 2^+-150 (zeros aside), and
+// those with a temperature below 2^-4 to 2^-5 of the largest, which would be held in fewer bits than in FP64 (57 below
+// the largest; a node a million times as hot cost the others' second derivatives seven digits).  The latter are
+// found in the conversion and left for the nodes' pass: a minimum beside the maxima, or a branch at the conversion's
+// barrier, took 2 to 6% of the kernels.
+__device__ __forceinline__ bool lift_cold(double T, unsigned mag) { return (mag >> 20) > (fx_mag(T) >> 20) + 4u; }
+__device__ __forceinline__ bool lift_fits(const unsigned* mag) {
+  const unsigned lowest = (1022u - 150u) << 20, highest = (1022u + 150u) << 20;
+  bool ok = true;
+#pragma unroll
+  for (int v = 0; v < 4; ++v) ok = ok && mag[v] < highest && (mag[v] == 0u || mag[v] > lowest);
+  return ok;
+}
+
 // u, v, w, T in FP64 to X [4][n3], and the derivatives of the lines of all directions to Y [3][4][n3] (elements whose
 // values do not fit one scale): the FP64 kernel's sums, by the block
 template <int NP, int NT>
@@ -136,9 +150,10 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
   fx64* const Y = reinterpret_cast<fx64*>(smem_raw);           // [3][4][n3]: derivatives
   FxDig* const X = reinterpret_cast<FxDig*>(Y + 12 * n3);      // [4][n3]: u, v, w, T
   __shared__ unsigned mag[4];
-  __shared__ int es[12];
+  __shared__ int es[12], cold;
   const int e = blockIdx.x, tid = threadIdx.x;
   if (tid < 4) mag[tid] = 0u;
+  if (tid == 0) cold = 0;
   if (tid < 12) es[tid] = E2S[(size_t)e * 12 + tid];
   __syncthreads();
   const double* const Pe = Pvol + (size_t)e * 7 * n3;
@@ -176,16 +191,16 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
   }
   __syncthreads();
   const float* const ml = MetL + (size_t)e * kMetL;
-  bool ok = ml[0] < 200.f;
-#pragma unroll
-  for (int v = 0; v < 4; ++v) ok = ok && mag[v] < ((1022u + 150u) << 20);
+  bool ok = ml[0] < 200.f && lift_fits(mag);
   if (ok) {
 #pragma unroll
     for (int it = 0; it < NPT; ++it) {
       const int node = tid + it * NT;
-      if (node < n3)
+      if (node < n3) {
 #pragma unroll
         for (int v = 0; v < 4; ++v) X[v * n3 + vsw<NP>(node)] = fd_from(x[it][v], fx_r0(57 - fx_exp(mag[v])));
+        if (lift_cold(x[it][3], mag[3])) cold = 1;
+      }
     }
     __syncthreads();
     // ---- derivatives.  |x| < 2^57 and |D| < 2^58 in digits: a sum of at most 5 products of (x_l +- x_(N-l)) and D
@@ -253,7 +268,9 @@ k_lift_fx(const double* __restrict__ Pvol, const double* __restrict__ Met, const
       }
     }
     __syncthreads();
-  } else {
+    ok = cold == 0;
+  }
+  if (!ok) {
     double* const Yd = reinterpret_cast<double*>(Y);
     lift_lines_fp64<NP, NT>(Pe, D, Yd + 12 * n3, Yd);
     lift_nodes_fp64<NP, NT>(Me, Yd);

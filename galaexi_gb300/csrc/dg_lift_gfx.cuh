@@ -117,10 +117,11 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
   int* const off = reinterpret_cast<int*>(J + n3);         // [3][2][n2]: the face nodes' places on their sides
   __shared__ unsigned mag[4], magY[4], magF[4];
   __shared__ LiftGfxScale sc[4];
-  __shared__ int es[12];
+  __shared__ int es[12], cold;
   __shared__ FxDig Lh[NP];
   const int e = blockIdx.x, tid = threadIdx.x;
   if (tid < 4) mag[tid] = magY[tid] = magF[tid] = 0u;
+  if (tid == 4) cold = 0;
   if (tid < 12) es[tid] = E2S[(size_t)e * 12 + tid];
   if (tid >= 32 && tid < 32 + n) Lh[tid - 32] = gb.Lh[tid - 32];
   __syncthreads();
@@ -164,8 +165,7 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
     for (int v = 0; v < 4; ++v) fx_block_max(m[v], &mag[v]);
   }
   __syncthreads();
-#pragma unroll
-  for (int v = 0; v < 4; ++v) ok = ok && mag[v] < ((1022u + 150u) << 20);
+  ok = ok && lift_fits(mag);
   // Scales (powers of two): |x| < 2^57, |M| < 2^58 and SurfElem n < 2^58 for each component of the gradient (in flat
   // elements they differ by the aspect ratio), |sJ| < 2^59; y = D x below 2^60 (as in
   // k_lift_fx), F = (SurfElem/2 n) dx below 2^59.  From here on the scale follows the largest |y| and |F| of the
@@ -182,7 +182,9 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         fx64* const x = X + v * n3 + vsw<NP>(node);
-        *x = fd_pack(fd_from(__longlong_as_double(*x), r0[v]));
+        const double d = __longlong_as_double(*x);
+        if (v == 3 && lift_cold(d, mag[3])) cold = 1;
+        *x = fd_pack(fd_from(d, r0[v]));
       }
     // ---- face fluxes, and the BR2 weights of the lines
     unsigned mf[4] = {0u, 0u, 0u, 0u}, my[4] = {0u, 0u, 0u, 0u};
@@ -318,9 +320,10 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
       }
     }
     __syncthreads();
+    ok = cold == 0;
     // ---- node by node
 #pragma unroll 1
-    for (int node = tid; node < n3; node += NT) {
+    for (int node = ok ? tid : n3; node < n3; node += NT) {
       const int i = node % n, j = (node / n) % n, k = node / n2, sn = vsw<NP>(node);
       const int ix[3] = {i, j, k}, ab[3] = {j + n * k, i + n * k, i + n * j};
       FxDig M[9];
@@ -371,7 +374,8 @@ k_lift_gfx(const double* __restrict__ Pvol, const double* __restrict__ Met, cons
         }
       }
     }
-  } else {
+  }
+  if (!ok) {
     lift_gen_fp64<NP, GAUSS, BR2, NT>(Pe, Me, Pf, Fgeo, es, nSides, basis.D, basis.Lhm, basis.Lhp,
                                       Gvol + (size_t)e * 15 * n3, reinterpret_cast<double*>(X),
                                       reinterpret_cast<double*>(F), reinterpret_cast<double*>(Y));
