@@ -89,10 +89,11 @@ int cfg_lift_lines() {
 }
 
 // FP64 weak form: the fixed-point kernel from N = 3 on (48^3 Euler, N = 3: 1.16 against 1.84 ms).  At N = 2 a block's
-// 27 nodes leave it waiting for its scales: it is the faster one (Navier-Stokes, 4^3 elements 16 against 22 us, 12^3
-// 33 against 37) only as long as the SMs hold all elements at once, kWeakFxResident blocks each; then 16^3 elements
-// take 59 against 53 us, 64^3 2.97 against 2.65 ms
-constexpr int kWeakFxResident = 10;
+// 27 nodes leave it waiting for its scales: it is the faster one on small meshes, up to kWeakFxResident elements per
+// SM.  One evaluation, Gauss nodes, Navier-Stokes, on 152 SMs, fixed point against FP64: 1728 elements 78.1 and 86.1
+// us, 2744 108.6 and 118.6, 3375 126.2 and 129.0, 4096 143.1 and 139.2 (Euler 34.9 and 39.0, 46.4 and 49.2, 51.3 and
+// 51.3, 57.4 and 53.4); the kernel alone with 64^3 elements 2.97 and 2.65 ms
+constexpr int kWeakFxResident = 22;
 template <typename R>
 constexpr bool weak_fx() { return std::is_same<R, double>::value && NP >= 3; }
 
@@ -200,8 +201,9 @@ void rhs_front(dg_ctx* ctx, PrecData<R>& P, const S* U, const gx::Gas<R>& gas, c
     }
   }
   if constexpr (EPB > 1 && std::is_same<S, double>::value) {
-    // fewer blocks than SMs: one element per block (4^3 elements, N = 2: 11.5 against 16.4 us; 8^3, N = 3: 12.7 against
-    // 14.9; at 10^3, N = 3, the two are equal)
+    // fewer blocks than SMs: one element per block (FP64 form, 4^3 elements, N = 2: 11.5 against 16.4 us; 8^3, N = 3:
+    // 12.7 against 14.9; at 10^3, N = 3, the two are equal.  Mixed form, a whole step on Gauss nodes: 4^3, N = 2: 154
+    // against 164 us, 8^3, N = 3: 134 against 144, 6^3, N = 4: 146 against 154)
     if (!persistent && grid < ctx->sms) {
       gx::k_prolong<NP, R, S, 1><<<ctx->nElems, gx::ProlongThreads<NP, 1>::v, 0, st>>>(U, ctx->E2S.p, bd.Lm, bd.Lp, gas, L,
                                                                                       P.Pvol.p, P.Uf.p, P.Pf.p);

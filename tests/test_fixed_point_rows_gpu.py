@@ -218,3 +218,32 @@ def test_hot_node(form):
     cold = np.s_[3, 1:, 1:, 1:, 4]
     err = np.linalg.norm(g[cold] - o[cold]) / np.linalg.norm(o[cold])
     assert err <= 5e-14, err
+
+
+@pytest.mark.parametrize("parab", [False, True], ids=["euler", "ns"])
+@pytest.mark.parametrize("form", ["pi", "kg", "weak"])
+def test_velocities_near_zero(form, parab):
+    """Velocities of 1e-25 ahead of a disturbance: the mass row and, for the Euler equations, the energy row are linear
+    in them (the others are the round-off of the constant pressure and temperature).  The oracle is within 2.1e-15 of 80
+    bits there."""
+    kw = FORMS[form]
+    m = mesh(5, kw, (2, 2, 1))
+    x = m.Elem_xGP
+    vel = 1e-25 * np.stack([np.sin(x[..., 0] + x[..., 1]), np.cos(x[..., 2]), np.sin(x[..., 1])], -1)
+    U = conservative(np.ones(x.shape[:4]), vel, np.full(x.shape[:4], 1 / 1.4))
+    g, o = both(gx.config(N=5, R=R, **(dict(kw, parabolic=True, mu0=1e-3) if parab else kw)), m, U)
+    r = rows(g, o)
+    assert max(r[0], 0.0 if parab else r[4]) <= 5e-14, r
+
+
+# largest meshes of the fixed-point weak kernel at N = 2 (22 elements per SM), one element more, and more than that
+@pytest.mark.parametrize("elements", [22, 23])
+@pytest.mark.parametrize("form", ["weak", "gauss"])
+def test_weak_form_at_n2_on_both_sides_of_its_rule(form, elements):
+    """Bar: the FP64 form's 1e-12 over all rows."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    kw = FORMS[form]
+    m = mesh(2, kw, (elements, sms // 8, 8))
+    U = noisy(m, "rule%s%d" % (form, elements), (2 * math.pi,) * 3)
+    g, o = both(gx.config(N=2, R=R, parabolic=True, mu0=1e-3, **kw), m, U)
+    assert np.linalg.norm(g - o) <= 1e-12 * np.linalg.norm(o)
