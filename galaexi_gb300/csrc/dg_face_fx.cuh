@@ -88,18 +88,17 @@ __device__ __forceinline__ void riemann_dp(const double dm[3], const FaceSide& L
     const bool superL = dp_ge0(Sl), superR = dp_le0(Sr);
     const bool left = superL || (!superR && dp_ge0(Ss));
     const double rho = left ? L.rho : R.rho, p = left ? L.p : R.p, us = left ? L.un : R.un;
-    const double es = left ? L.E * L.srho : R.E * R.srho, E = left ? L.E : R.E, mn = left ? mnL : mnR, S = left ? Sl : Sr;
-    const double fac = dp_div(mn, S - Ss), dus = Ss - us;
-    const double Est = es + dus * (Ss + dp_div(p, mn));
-    const double Se = superL || superR ? 0. : S;
-    const double m = rho * us;
-    const double m0 = superL || superR ? m : m + Se * (fac - rho);
-    const double pn = superL || superR ? p : p + Se * (fac * dus);
-    F[0] = m0;
+    const double E = left ? L.E : R.E, S = left ? Sl : Sr;
+    // with k = (Ss - u) / (S - Ss) the star state's jumps are U* - U = k U + ..., without the difference of two states:
+    //   rho* = rho (1 + k),  S (E* - E) = S k (E + p) + S rho* (Ss - u) Ss
+    const bool super = superL || superR;
+    const double dus = Ss - us, k = dus * dp_rcp(S - Ss);
+    const double ust = super ? us : fma(S, k, us), b = super ? 0. : S * (fma(rho, k, rho) * dus);
+    F[0] = rho * ust;
+    const double pn = p + b;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) F[1 + k] = (left ? L.v[k] : R.v[k]) * m0 + pn * n[k];
-    const double fe = (E + p) * us;
-    F[4] = superL || superR ? fe : fe + Se * (fac * Est - E);
+    for (int c = 0; c < 3; ++c) F[1 + c] = (left ? L.v[c] : R.v[c]) * F[0] + pn * n[c];
+    F[4] = (E + p) * ust + (super ? 0. : b * Ss);
     return;
   }
   central_flux<CENTRAL>(L, R, n, HL, HR, F);
