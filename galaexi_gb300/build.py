@@ -1,6 +1,6 @@
 """Build the galaexi_gb300 shared library (CUDA for sm_103a + host C++), in-tree.
 
-Two translation units per polynomial degree (dg_np<N+1>.cu, dg_fx<N+1>.cu) plus the C-ABI and host files are
+Two translation units per polynomial degree (dg_np<N+1>.cu; dg_fx<N+1>.cu from N = 2 on) plus the C-ABI and host files are
 compiled in parallel with nvcc and linked into galaexi_gb300/_build/libgalaexi_gb300.so.
 """
 import concurrent.futures
@@ -20,7 +20,7 @@ CUFLAGS = ARCH + ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xco
 
 def sources():
     srcs = ["dg_api.cu", "dg_host.cpp", "dg_hdf5.cpp", "dg_hopr.cpp", "dg_noalloc.cu", "dg_face_fx.cu", "dg_fx_mesh.cu"] + [
-        "dg_np%d.cu" % np_ for np_ in range(2, 11)] + ["dg_fx%d.cu" % np_ for np_ in range(2, 11)]
+        "dg_np%d.cu" % np_ for np_ in range(2, 11)] + ["dg_fx%d.cu" % np_ for np_ in range(3, 11)]
     return [os.path.join(CSRC, s) for s in srcs]
 
 

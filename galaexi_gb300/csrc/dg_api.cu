@@ -55,9 +55,9 @@ const gxc::NPTable* table_for(int n) {
   return nullptr;
 }
 
+// (none for N = 1)
 const gxc::FxTable* fx_table_for(int n) {
   switch (n) {
-    case 2: return &gx_fx_table_2;
     case 3: return &gx_fx_table_3;
     case 4: return &gx_fx_table_4;
     case 5: return &gx_fx_table_5;
@@ -517,7 +517,8 @@ int dg_ctx_create(const dg_config* cfg, dg_ctx** out) {
     ctx->sms = 0;
   if (rc == DG_OK) rc = (cfg->precision == DG_PRECISION_FP64) ? T->configure_d() : T->configure_f();
   if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64) rc = upload_fx_basis(ctx);
-  if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64) rc = fx_table_for(ctx->n)->configure(ctx);
+  if (const gxc::FxTable* F = fx_table_for(ctx->n))
+    if (rc == DG_OK && cfg->precision == DG_PRECISION_FP64) rc = F->configure(ctx);
   if (rc == DG_OK && !(ctx->red.alloc(2) && ctx->bad.alloc(1) && ctx->kerr.alloc(1))) { set_error("cudaMalloc"); rc = DG_ERR_ALLOC; }
   if (rc == DG_OK && cudaMemset(ctx->kerr.p, 0, sizeof(int)) != cudaSuccess) { set_error("clear error flag"); rc = DG_ERR_CUDA; }
   if (rc == DG_OK && !fmat.empty()) {

@@ -190,7 +190,7 @@ struct NPTable {
   int (*relift)(dg_ctx*, cudaStream_t st);
 };
 
-// the fixed-point kernels of the FP64 form, in translation units of their own (dg_fx<NP>.cu)
+// the fixed-point kernels of the FP64 form, in translation units of their own (dg_fx<NP>.cu, from N = 2 on)
 struct FxTable {
   int (*configure)(const dg_ctx*);
   // volume kernel of the weak form and of the split forms PI and KG (Gauss-Lobatto nodes)
@@ -213,7 +213,7 @@ bool face_dp(const dg_ctx* ctx, const gx::Gas<double>& gas, cudaStream_t st);
 #define GX_DECLARE_NP(NPV)                   \
   extern const gxc::NPTable gx_np_table_##NPV; \
   extern const gxc::FxTable gx_fx_table_##NPV;
-GX_DECLARE_NP(2)
+GX_DECLARE_NP(2)  // (gx_fx_table_2: the name only, for the discarded branches of dg_np2.cu)
 GX_DECLARE_NP(3)
 GX_DECLARE_NP(4)
 GX_DECLARE_NP(5)

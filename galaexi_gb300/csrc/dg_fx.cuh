@@ -139,7 +139,6 @@ struct FxDig {
   int h, l;
 };
 __device__ __forceinline__ FxDig fd_split(fx64 x) { return {(int)(x >> 30), (int)x & 0x3fffffff}; }
-__device__ __forceinline__ fx64 fd_join(FxDig a) { return ((fx64)a.h << 30) + a.l; }
 __device__ __forceinline__ FxDig operator+(FxDig a, FxDig b) { return {a.h + b.h, a.l + b.l}; }
 __device__ __forceinline__ FxDig operator-(FxDig a, FxDig b) { return {a.h - b.h, a.l - b.l}; }
 struct FxDot {

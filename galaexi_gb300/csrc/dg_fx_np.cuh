@@ -127,14 +127,11 @@ int volume_spl(dg_ctx* ctx, const double* U, const gx::Gas<double>& gas, gx::RKA
 }
 
 int volume(dg_ctx* ctx, const double* U, const gx::Gas<double>& gas, gx::RKArgs rk, int rkmode, cudaStream_t st) {
-  if (ctx->cfg.split_dg == DG_SPLIT_NONE) {
-    if constexpr (NP >= 3) return volume_weak(ctx, U, gas, rk, rkmode, st);
+  switch (ctx->cfg.split_dg) {
+    case DG_SPLIT_NONE: return volume_weak(ctx, U, gas, rk, rkmode, st);
+    case DG_SPLIT_KG: return volume_spl<DG_SPLIT_KG>(ctx, U, gas, rk, rkmode, st);
+    default: return volume_spl<DG_SPLIT_PI>(ctx, U, gas, rk, rkmode, st);
   }
-  if constexpr (NP >= 3)
-    return ctx->cfg.split_dg == DG_SPLIT_KG ? volume_spl<DG_SPLIT_KG>(ctx, U, gas, rk, rkmode, st)
-                                            : volume_spl<DG_SPLIT_PI>(ctx, U, gas, rk, rkmode, st);
-  gxh::set_error("split form needs N >= 2");
-  return DG_ERR_UNSUPPORTED;
 }
 
 template <int SPL>
@@ -205,42 +202,35 @@ void lift_general(dg_ctx* ctx, cudaStream_t st) {
 }
 
 void lift(dg_ctx* ctx, cudaStream_t st) {
-  if constexpr (NP >= 3) {
-    if (ctx->cfg.node_type == DG_NODETYPE_GAUSS || ctx->cfg.lifting == DG_LIFTING_BR2) return lift_general(ctx, st);
-    gxc::PrecData<double>& P = ctx->d;
-    const auto& lb = kept<gx::LiftFxBasis<NP>>(ctx->fx_lift, [&](gx::LiftFxBasis<NP>& b) { lift_basis(ctx, b); });
-    auto kern = ctx->face_exact ? gx::k_lift_fx<NP, true> : gx::k_lift_fx<NP, false>;
-    kern<<<ctx->nElems, gx::LiftFx<NP>::NT, gx::LiftFx<NP>::smem, st>>>(
-        P.Pvol.p, P.Met.p, ctx->MetL.p, P.Pf.p, P.Fgeo.p, ctx->E2S.p, lb, P.basis.p, ctx->B.Lhm[0], ctx->nSides, P.Gvol.p,
-        P.Gf.p);
-  }
+  if (ctx->cfg.node_type == DG_NODETYPE_GAUSS || ctx->cfg.lifting == DG_LIFTING_BR2) return lift_general(ctx, st);
+  gxc::PrecData<double>& P = ctx->d;
+  const auto& lb = kept<gx::LiftFxBasis<NP>>(ctx->fx_lift, [&](gx::LiftFxBasis<NP>& b) { lift_basis(ctx, b); });
+  auto kern = ctx->face_exact ? gx::k_lift_fx<NP, true> : gx::k_lift_fx<NP, false>;
+  kern<<<ctx->nElems, gx::LiftFx<NP>::NT, gx::LiftFx<NP>::smem, st>>>(
+      P.Pvol.p, P.Met.p, ctx->MetL.p, P.Pf.p, P.Fgeo.p, ctx->E2S.p, lb, P.basis.p, ctx->B.Lhm[0], ctx->nSides, P.Gvol.p,
+      P.Gf.p);
 }
 
 int configure(const dg_ctx* ctx) {
-  if constexpr (NP >= 3)
-    if (ctx->cfg.split_dg == DG_SPLIT_NONE) {
-      int rc = smem_attr(gx::k_volume_wfx<NP, 0>, gx::VolWfx<NP>::smem, "k_volume_wfx attributes");
-      if (rc == DG_OK) rc = smem_attr(gx::k_volume_wfx<NP, 1>, gx::VolWfx<NP>::smem, "k_volume_wfx attributes");
-      if (rc != DG_OK) return rc;
-    }
-  if constexpr (NP >= 3)
-    if (ctx->cfg.parabolic) {
-      const bool gauss = ctx->cfg.node_type == DG_NODETYPE_GAUSS, br2 = ctx->cfg.lifting == DG_LIFTING_BR2;
-      int rc = DG_OK;
-      if (!gauss && br2) rc = smem_attr(gx::k_lift_gfx<NP, false, true>, gx::LiftGfx<NP>::smem, "k_lift_gfx attributes");
-      else if (br2) rc = smem_attr(gx::k_lift_gfx<NP, true, true>, gx::LiftGfx<NP>::smem, "k_lift_gfx attributes");
-      else if (gauss) rc = smem_attr(gx::k_lift_gfx<NP, true, false>, gx::LiftGfx<NP>::smem, "k_lift_gfx attributes");
-      else {
-        rc = smem_attr(gx::k_lift_fx<NP, true>, gx::LiftFx<NP>::smem, "k_lift_fx attributes");
-        if (rc == DG_OK) rc = smem_attr(gx::k_lift_fx<NP, false>, gx::LiftFx<NP>::smem, "k_lift_fx attributes");
-      }
-      if (rc != DG_OK) return rc;
-    }
-  if constexpr (NP >= 3) {
-    if (ctx->cfg.split_dg == DG_SPLIT_PI) return configure_spl<DG_SPLIT_PI>();
-    if (ctx->cfg.split_dg == DG_SPLIT_KG) return configure_spl<DG_SPLIT_KG>();
+  const dg_config& c = ctx->cfg;
+  int rc = DG_OK;
+  if (c.split_dg == DG_SPLIT_NONE) {
+    rc = smem_attr(gx::k_volume_wfx<NP, 0>, gx::VolWfx<NP>::smem, "k_volume_wfx attributes");
+    if (rc == DG_OK) rc = smem_attr(gx::k_volume_wfx<NP, 1>, gx::VolWfx<NP>::smem, "k_volume_wfx attributes");
   }
-  return DG_OK;
+  if (rc == DG_OK && c.parabolic) {
+    const bool gauss = c.node_type == DG_NODETYPE_GAUSS, br2 = c.lifting == DG_LIFTING_BR2;
+    if (!gauss && br2) rc = smem_attr(gx::k_lift_gfx<NP, false, true>, gx::LiftGfx<NP>::smem, "k_lift_gfx attributes");
+    else if (br2) rc = smem_attr(gx::k_lift_gfx<NP, true, true>, gx::LiftGfx<NP>::smem, "k_lift_gfx attributes");
+    else if (gauss) rc = smem_attr(gx::k_lift_gfx<NP, true, false>, gx::LiftGfx<NP>::smem, "k_lift_gfx attributes");
+    else {
+      rc = smem_attr(gx::k_lift_fx<NP, true>, gx::LiftFx<NP>::smem, "k_lift_fx attributes");
+      if (rc == DG_OK) rc = smem_attr(gx::k_lift_fx<NP, false>, gx::LiftFx<NP>::smem, "k_lift_fx attributes");
+    }
+  }
+  if (rc == DG_OK && c.split_dg == DG_SPLIT_PI) rc = configure_spl<DG_SPLIT_PI>();
+  if (rc == DG_OK && c.split_dg == DG_SPLIT_KG) rc = configure_spl<DG_SPLIT_KG>();
+  return rc;
 }
 
 }  // namespace

@@ -233,7 +233,7 @@ void rhs_front(dg_ctx* ctx, PrecData<R>& P, const S* U, const gx::Gas<R>& gas, c
         lines = true;
       }
     }
-    if constexpr (std::is_same<R, double>::value && V0 == 1) {
+    if constexpr (std::is_same<R, double>::value && V0 == 1 && NP >= 3) {
       // FP64 form in strong non-conservative form: fixed point
       if (ctx->lift_fx) {
         GX_CAT(gx_fx_table_, GX_NP).lift(ctx, st);

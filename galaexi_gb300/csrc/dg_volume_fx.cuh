@@ -46,10 +46,6 @@ template <int NP> struct VolFx {
     return sizeof(fx64) * (size_t)(6 + 3 * dslots(parab)) * NP * NP * NP;
   }
 };
-template <int NP, typename R, int SPLIT, typename S> struct UseVolFx {
-  static constexpr bool v = std::is_same<R, double>::value && std::is_same<S, double>::value && NP >= 3 &&
-                            (SPLIT == DG_SPLIT_PI || SPLIT == DG_SPLIT_KG);
-};
 // what the kernel needs of the basis: limbs of Q(i,l) 2^62 at [l + n i] and of w_0/w_i 2^60
 template <int NP> struct VolFxBasis {
   FxLimb Q[NP * NP], iw[NP];
