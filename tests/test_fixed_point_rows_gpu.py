@@ -247,3 +247,41 @@ def test_weak_form_at_n2_on_both_sides_of_its_rule(form, elements):
     U = noisy(m, "rule%s%d" % (form, elements), (2 * math.pi,) * 3)
     g, o = both(gx.config(N=2, R=R, parabolic=True, mu0=1e-3, **kw), m, U)
     assert np.linalg.norm(g - o) <= 1e-12 * np.linalg.norm(o)
+
+
+@pytest.mark.parametrize("form", list(FORMS))
+@pytest.mark.parametrize("N,units", [(2, 1e-4), (4, 1e5), (7, 1e-6), (9, 1e2)])
+def test_rows_in_other_units(N, units, form):
+    """Lengths in `units`, velocities in sqrt(units), density in 1/units: the rows lie powers of the units apart.
+    The oracle is within 5.2e-14 of 80 bits in the mass and energy rows and 8.5e-13 in the momentum rows (Gauss nodes,
+    N = 9: 3.4e-12); bars four to five times that."""
+    kw = FORMS[form]
+    L, V, D = units, math.sqrt(units), 1.0 / units
+    m = mesh(N, kw, (2, 2, 1), (2 * math.pi * L,) * 3)
+    m1 = mesh(N, kw, (2, 2, 1))
+    U = noisy(m1, "rows%d%s" % (N, form), (2 * math.pi,) * 3) * np.array([D, D * V, D * V, D * V, D * V * V])
+    g, o = both(gx.config(N=N, R=R, parabolic=True, mu0=2e-3 * D * V * L, **kw), m, U)
+    r = rows(g, o)
+    assert max(r[0], r[4]) <= 2.5e-13 and max(r[1:4]) <= (1.5e-11 if N == 9 and "gauss" in form else 4e-12), r
+
+
+# (a pressure contrast has inadmissible traces on Gauss nodes)
+@pytest.mark.parametrize("form,what", [(f, w) for f in FORMS for w in ("density", "pressure")
+                                       if w == "density" or "gauss" not in f])
+@pytest.mark.parametrize("N", [3, 6])
+def test_rows_of_refused_elements(N, form, what):
+    """An element with a contrast of 2000 in density (with the momenta and the energy) or pressure among ordinary ones.
+    The oracle is within 1.1e-15 of 80 bits, 2.9e-13 in the momentum row of the vanishing velocity; bars nine and seven
+    times that."""
+    kw = dict(FORMS[form], Riemann="lf")
+    m = mesh(N, kw, (3, 2, 1))
+    U = noisy(m, "refused" + form, (2 * math.pi,) * 3)
+    s = bump(m, 1)[..., None]
+    if what == "density":
+        U[1] *= 2000.0 ** s
+    else:
+        U[1, ..., 4:] *= 2000.0 ** s
+    g, o = both(gx.config(N=N, R=R, parabolic=True, mu0=2e-3, **kw), m, U)
+    assert np.isfinite(o).all()
+    r = rows(g, o)
+    assert max(r[0], r[1], r[2], r[4]) <= 1e-14 and r[3] <= 2e-12, r
