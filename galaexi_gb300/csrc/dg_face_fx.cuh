@@ -70,7 +70,8 @@ __device__ __forceinline__ void riemann_dp(const double dm[3], const FaceSide& L
   double rr = L.rho * R.rho;
   // (two negative densities: no square root)
   rr = __hiloint2double(__double2hiint(rr) | (__double2hiint(L.rho) & (int)0x80000000), __double2loint(rr));
-  const double rt = dp_sqrt(rr);
+  // (a product outside the helpers' range: the roots one by one, densities of 1e-150 or 1e150 would leave FP64's)
+  const double rt = dp_exponent_in(rr, 123, 1800) ? dp_sqrt(rr) : dp_sqrt_rare(L.rho) * dp_sqrt_rare(R.rho);
   const double w = R.rho * dp_rcp(R.rho + rt);
   const double un = fma(w, R.un - L.un, L.un);
   double u[3];
