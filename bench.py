@@ -43,17 +43,19 @@ ALG_BYTES_N7 = 510.0  # compulsory HBM bytes per DOF-stage of a fully fused impl
 #       -k regex:<kernel> -s 3 -c 1 python bench.py [--precision mixed] --workload tgv_n7_16cube_split_pi_roe_br1
 #       --steps 2 --warmup 1 --no-e2e --no-cpu-baseline --no-profile --no-extras
 #   and for k_volume_fx (FP64) the executed DFMA + DADD + DMUL thread-instructions
-#   (sm__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum).
-CAPTURE = {"fp64": "ncu, one launch of each kernel, tgv_n7_16cube, 2026-12-05 06:50 UTC, commit d6347c9",
+#   (sm__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum) and the warp instructions (smsp__inst_executed.sum).
+CAPTURE = {"fp64": "ncu, one launch of each kernel, tgv_n7_16cube, 2026-12-05 09:45 UTC, commit a0ac1b5",
            "mixed": "ncu, one kernel and one launch per capture, tgv_n7_16cube, 2026-12-04 20:25 UTC, commit c00486e"}
 _DOF16 = 2097152
 DRAM_BYTES_PER_DOF = {  # read + write per launch
-    "fp64": {"prolong": (84183040 + 196764928) / _DOF16, "lift": (285846784 + 338873600) / _DOF16,
-             "face": (289464320 + 24847616) / _DOF16, "volume": (670398208 + 145141760) / _DOF16},
+    "fp64": {"prolong": (84420864 + 197648128) / _DOF16, "lift": (285799168 + 299833344) / _DOF16,
+             "face": (289464064 + 24371200) / _DOF16, "volume": (670490880 + 145169664) / _DOF16},
     "mixed": {"prolong": (84130048 + 69619200) / _DOF16, "lift": (157313792 + 127674624) / _DOF16,
               "face": (144744960 + 9332992) / _DOF16, "volume": (427753216 + 123999744) / _DOF16},
 }
 KVOL_FP64_INSTR_PER_DOF = (50331648 + 10485760 + 37748736) / _DOF16
+KVOL_INST_PER_DOF = 312381440 / _DOF16  # warp instructions of the same capture (smsp__inst_executed.sum)
+ISSUE_PER_CYCLE = 4 * 152  # one warp instruction per scheduler: 4 schedulers, 152 SMs
 FP64_ISSUE_PER_CYCLE = 304  # sm__sass_thread_inst_executed_op_dfma_pred_on.sum.peak_sustained (152 SMs x 2)
 TGV_R = 71.42857
 CFL = 0.8  # CFLscale / DFLscale of the reference's TGV regression (regressioncheck/checks/tgv/split/parameter.ini)
@@ -679,26 +681,37 @@ def profile_roofline(args, op, U, dt, stream, nDOF, sm_mhz=None):
     nat.check(nat.lib().dg_measure_fma_peak(1, ctypes.byref(peak32)), "fma peak fp32")
     peak = peak64.value if args.precision == "fp64" else peak32.value
     vol_flops = ALG_FLOPS_N7["volume"] * nDOF
-    achieved = vol_flops / (kms["volume"] * 1e-3) * 1e-12
+    flop_rate = vol_flops / (kms["volume"] * 1e-3) * 1e-12
+    clock = (sm_mhz or 2070.0) * 1e6
     mp = measured_peaks()
     hbm_peak = mp.get("hbm_gbs", 6800.0)
     stage_s = kms["stage"] * 1e-3
     alg_b = ALG_BYTES_N7 if args.precision == "fp64" else ALG_BYTES_N7_MIXED
+    if args.precision == "fp64":
+        # the pair fluxes and contractions run as integer products (block fixed point): bound by the issue of warp
+        # instructions, an integer one holding its pipe for two cycles
+        bound = {"bound": "integer issue", "achieved": KVOL_INST_PER_DOF * nDOF / (kms["volume"] * 1e-3) * 1e-9,
+                 "peak": ISSUE_PER_CYCLE * clock * 1e-9, "unit": "G warp instructions/s",
+                 "peak_source": "4 schedulers x 152 SMs x the SM clock sampled in the timed region; instructions per DOF "
+                                "from a one-kernel capture"}
+    else:
+        bound = {"bound": "fp32", "achieved": flop_rate, "peak": peak * 1e-3, "unit": "TFLOP/s",
+                 "peak_source": "FMA-chain microkernel measured in this run (no FP32 CUDA-core peak in "
+                                "MEASURED_PEAKS.json)"}
     roofline = {
         "kernel": ("k_volume_fx" if args.precision == "fp64" else "k_volume_lines") +
                   " (split-form volume + viscous volume + surface integral + Jacobian + RK stage)",
-        "bound": "fp64" if args.precision == "fp64" else "fp32",
-        "achieved": achieved, "peak": peak * 1e-3, "unit": "TFLOP/s", "frac": achieved / (peak * 1e-3),
-        "peak_source": "FMA-chain microkernel measured in this run (no FP64/FP32 CUDA-core peak in MEASURED_PEAKS.json)",
+        **bound, "frac": bound["achieved"] / bound["peak"],
         "alg_flops_per_dof": ALG_FLOPS_N7["volume"],
+        # the algorithm's floating-point operations over the FMA peak of the form's type: above one in the FP64 form,
+        # whose products are not floating point
+        "alg_tflops": flop_rate, "alg_tflops_over_fma_peak": flop_rate / (peak * 1e-3),
         "traffic": DRAM_BYTES_PER_DOF[args.precision]["volume"] * nDOF,
         "traffic_source": "dram__bytes_read+write per DOF of one launch, scaled by nDOF (%s)" % CAPTURE[args.precision],
         # executed FP64 instructions (captured per DOF) over the FP64 issue capacity at the SM clock
         # sampled during the timed region
         "exec_fp64_issue_frac": (KVOL_FP64_INSTR_PER_DOF * nDOF / (kms["volume"] * 1e-3))
-                                / (FP64_ISSUE_PER_CYCLE * (sm_mhz or 2070.0) * 1e6) if args.precision == "fp64" else None,
-        "note": ("the pair fluxes and contractions of the FP64 form run as integer products (block fixed point), so the "
-                 "algorithmic rate exceeds the FP64 FMA peak") if args.precision == "fp64" else None,
+                                / (FP64_ISSUE_PER_CYCLE * clock) if args.precision == "fp64" else None,
         "kernel_ms": kms,
         "stage": {"alg_flops_per_dof_stage": sum(ALG_FLOPS_N7.values()),
                   "achieved_tflops": sum(ALG_FLOPS_N7.values()) * nDOF / stage_s * 1e-12,
