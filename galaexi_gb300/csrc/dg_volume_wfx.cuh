@@ -24,7 +24,8 @@ namespace gx {
 
 template <int NP> struct VolWfx {
   static constexpr int n3 = NP * NP * NP, work = n3 > 5 * NP * NP ? n3 : 5 * NP * NP;
-  static constexpr int NT = work >= 256 ? 256 : (work + 31) / 32 * 32;
+  // (n = 10: shared memory holds one block per SM)
+  static constexpr int NT = NP == 10 ? 512 : (work >= 256 ? 256 : (work + 31) / 32 * 32);
   static constexpr int MINB = 640 / NT > 16 ? 16 : 640 / NT;  // 96 registers per thread
   static constexpr size_t smem = sizeof(fx64) * 15 * n3;
 };
