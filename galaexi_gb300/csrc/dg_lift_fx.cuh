@@ -55,7 +55,8 @@ __device__ __forceinline__ bool lift_fits(const unsigned* mag) {
 }
 
 // u, v, w, T in FP64 to X [4][n3], and the derivatives of the lines of all directions to Y [3][4][n3] (elements whose
-// values do not fit one scale): the FP64 kernel's sums, by the block
+// values do not fit one scale): the FP64 kernel's sums, by the block (N = 7, 16^3, all elements: the kernel 0.590 ms, as
+// k_lift; node by node from global memory 0.773)
 template <int NP, int NT>
 __device__ __noinline__ void lift_lines_fp64(const double* Pe, const double* D, double* X, double* Y) {
   constexpr int n = NP, n2 = NP * NP, n3 = NP * NP * NP;

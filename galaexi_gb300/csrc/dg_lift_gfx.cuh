@@ -13,8 +13,8 @@
 // one thread per node adds up; one thread per line and variable prolongs to the line's two faces, again with
 // even and odd parts, which gives both traces for the products of one.  Bound by the integer pipes (issue 53%,
 // ALU 56% at N = 5 and 7; the conversions to integers on the FP64 pipe instead made it 4% slower).  k_lift and
-// now: N = 5, 24^3 curved, Gauss BR2 2.04 -> 0.611 ms; Gauss BR1 N = 2, 64^3 4.69 -> 2.39, N = 4, 32^3
-// 2.15 -> 0.845, N = 7, 20^3 2.20 -> 0.726, N = 9, 16^3 3.17 -> 0.907; Gauss-Lobatto BR2 N = 7, 24^3 2.75 -> 1.21.
+// now: N = 5, 24^3 curved, Gauss BR2 2.04 -> 0.629 ms; Gauss BR1 N = 2, 64^3 4.69 -> 2.43, N = 4, 32^3
+// 2.15 -> 0.851, N = 7, 20^3 2.20 -> 0.729, N = 9, 16^3 3.17 -> 0.919; Gauss-Lobatto BR2 N = 7, 24^3 2.75 -> 1.22.
 #pragma once
 #include "dg_fx.cuh"
 #include "dg_kernels.cuh"
@@ -24,7 +24,7 @@ namespace gx {
 
 template <int NP> struct LiftGfx {
   // threads: whole passes over the 12 n^2 lines and the n^3 nodes, and enough warps beside the shared memory (one
-  // thread for each of the 12 n^2 lines of small elements: N = 2 3.33 ms, N = 3, 48^3 2.59 against 1.45)
+  // thread for each of the 12 n^2 lines of small elements: N = 2 3.33 ms, N = 3, 48^3 2.59 against 1.48)
   static constexpr int NT = NP <= 4 ? 64 : (NP == 5 ? 160 : (NP == 6 ? 224 : (NP == 7 ? 352 : (NP == 8 ? 256 : 512))));
   static constexpr size_t smem = sizeof(fx64) * (17 * NP * NP * NP + 78 * NP * NP) + sizeof(int) * 6 * NP * NP;
   static constexpr int byreg = NT == 512 ? 1 : 704 / NT, bysm = (int)((227 * 1024) / (smem + 2048));
@@ -45,7 +45,8 @@ struct LiftGfxScale {
   int KY, KF, kG, s_o, kt, kb;
 };
 
-// The FP64 lifting by the block (elements whose values do not fit one scale): the gradients to Gvol, those that the
+// The FP64 lifting by the block (elements whose values do not fit one scale; FP64-issue bound like k_lift: all elements
+// of 20^3, N = 5, Gauss BR1 and BR2 0.91 and 1.16 ms, k_lift 1.01 and 1.19): the gradients to Gvol, those that the
 // traces are formed from (BR2: the volume part) to Y.  X, F: shared memory as in the kernel below
 template <int NP, bool GAUSS, bool BR2, int NT>
 __device__ __noinline__ void lift_gen_fp64(const double* Pe, const double* Me, const double* Pf, const double* Fgeo,

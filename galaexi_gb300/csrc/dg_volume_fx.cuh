@@ -178,7 +178,7 @@ __device__ __forceinline__ void vol_fx_scales(const unsigned* mag, const float* 
 }
 // largest magnitudes of an element's face fluxes into out[5 * direction + row].  Large blocks: a warp takes whole
 // groups, one reduction each (24^3, N = 7: the kernel 1.86 ms, 1.88 with every warp in all 15 reductions).  Small
-// blocks: all warps together, five loads in flight (64^3, N = 2: 1.94 against 2.46 ms).
+// blocks: all warps together, five loads in flight (64^3, N = 2, when it was written: 1.94 against 2.46 ms).
 template <int NP, int NT>
 __device__ __forceinline__ void vol_flux_max(const double* Flux, const int* es, unsigned* out) {
   constexpr int n2 = NP * NP, NW = NT / 32;
@@ -217,7 +217,9 @@ __device__ __forceinline__ void vol_flux_max(const double* Flux, const int* es, 
 // The same sums in FP64 by the block, in the operations of k_volume: for elements whose values do not fit one scale
 // per quantity (infinities and NaN, magnitudes outside 2^+-150, densities or pressures that differ by more than the
 // scales allow within the element, which one scale would hold less exactly than FP64).  Bound by the FP64 pipe like
-// k_volume, whose work it does: the viscous or weak fluxes once per node, each pair once.  SPLIT < 0: weak form.
+// k_volume, whose work it does: the viscous or weak fluxes once per node, each pair once (N = 7, 16^3, Navier-Stokes,
+// all elements: 2.13 ms, k_volume 1.95; weak form on Gauss nodes 1.17 and 0.98; node by node from global memory they
+// took 6.95 and 5.68).  SPLIT < 0: weak form.
 // A: the block's shared memory, of which the fixed-point values are not needed any more (SPLIT < 0: 15 slots, else
 // 27, or 21 for the Euler equations); the results are left there as [node][5].  D: n^2 words for the split form's
 // matrix (the limbs' place: with words of its own the block of n = 4 fits an SM 14 instead of 15 times).

@@ -13,7 +13,7 @@
 // contracts the line with D_hat in even and odd parts (it is centro-antisymmetric), adds the line's two face
 // fluxes with their L_hat the same way, and puts the results in the fluxes' place; the three directions' results
 // of a node are integers of one scale and are added up exactly.  24^3 curved, N = 5, Gauss, Navier-Stokes: 1.29 ms
-// before, 0.905 ms; 48^3 Euler, N = 3: 1.84 and 1.17 ms.  With one scale for all rows and directions 0.87 and
+// before, 0.905 ms; 48^3 Euler, N = 3: 1.84 and 1.19 ms.  With one scale for all rows and directions 0.87 and
 // 1.04 ms, but on flat elements (1:100) the errors of the smallest row grew to 95 times the FP64 kernel's.
 #pragma once
 #include "dg_fx.cuh"
@@ -24,7 +24,7 @@ namespace gx {
 
 template <int NP> struct VolWfx {
   static constexpr int n3 = NP * NP * NP, work = n3 > 5 * NP * NP ? n3 : 5 * NP * NP;
-  // (n = 10: shared memory holds one block per SM)
+  // (n = 10: shared memory holds one block per SM; 12^3, Gauss, Navier-Stokes 0.667 ms with 256 threads, 0.551 with 512)
   static constexpr int NT = NP == 10 ? 512 : (work >= 256 ? 256 : (work + 31) / 32 * 32);
   static constexpr int MINB = 640 / NT > 16 ? 16 : 640 / NT;  // 96 registers per thread
   static constexpr size_t smem = sizeof(fx64) * 15 * n3;
